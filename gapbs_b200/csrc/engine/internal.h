@@ -43,6 +43,26 @@ struct BinConfig {
   int min_len[kNumBins] = {4096, 128, 64, 32, 16, 8, 1, 0};
 };
 
+// Warp tasks of the rows of one CSR for a resident solve (resident.h): rows
+// by descending length, position p being row order[p] (p itself when order
+// is null), those of at least `segment` entries cut into segments of as many.
+// A resident solve gathers the contribs of the first kResidentTile vertices,
+// the highest in-degrees, from shared memory (160 KB; with 192 KB Kronecker
+// graphs of 2^20 vertices gain 2 %, uniform ones of 2^22 lose 3 % and larger
+// ones up to 40 %: their gathers in flight need the L1 space).
+constexpr int kResidentTile = 40960;
+struct RowTasks {
+  bool ready = false;
+  int32_t segment = 0;
+  int32_t row_start[kNumBins + 1] = {};   // first position of bin b
+  int32_t task_start[kNumBins + 1] = {};  // first task of bin b; bin 0: segments
+  int32_t *order = nullptr;
+  int4 *seg = nullptr;           // segment -> (row, the row's first segment, first entry, end)
+  float *seg_partial = nullptr;  // per segment
+  unsigned *ticket = nullptr;    // per segment; a row's is at its first
+};
+void FreeRowTasks(RowTasks *r);
+
 struct DeviceGraph {
   int64_t n = 0, m = 0;
   bool directed = false;
@@ -74,6 +94,10 @@ struct DeviceGraph {
   int32_t *seg_first = nullptr;   // hub row -> first segment (num_hub_rows+1)
   unsigned *hub_ticket = nullptr; // per hub row
   float *seg_partial = nullptr;   // per segment
+  // tasks of the resident solves over the in-rows and (directed: adjoint)
+  // the out-rows, built by the first such solve
+  RowTasks in_tasks, out_tasks;
+  int64_t tile_entries = 0;  // in-entries of the first kResidentTile vertices
 };
 
 // Per-solve convergence control, in device memory.
@@ -90,7 +114,7 @@ struct Scratch {
   float *base = nullptr;       // per-vertex (1-d) t (PPR), new ids
   float *outbuf = nullptr;     // n x ncols scores in original ids
   float *tele = nullptr;       // teleport staging (original ids)
-  float *aux[2] = {nullptr, nullptr};  // adjoint: forward scores (new ids), staging
+  float *aux = nullptr;        // adjoint: forward scores staging (original ids)
   float *edge_buf = nullptr;   // adjoint: m edge gradients (device staging)
   double *norm = nullptr;      // adjoint: ||w||_1
   int64_t cap_edges = 0;
@@ -230,15 +254,10 @@ cudaError_t LaunchPullInit(const DeviceGraph &g, Scratch &sc, const float *tele_
                            float init_scalar, float damping, cudaStream_t s);
 // Kernel to run for one sweep of `a` (a function pointer for LoopGraph).
 const void *PullSweepKernel(const PullArgs &a);
-// Warp-per-row sweep over an arbitrary (unsorted) CSR given in a.rowoff /
-// a.col, a.nblocks blocks, grid-stride; used for adjoint sweeps over the
-// out-rows of directed graphs.
-const void *PullGenericKernel(const PullArgs &a);
 // Per-edge weight gradient and teleport gradient of the adjoint (pull.cu).
-cudaError_t LaunchAdjointGrads(const DeviceGraph &g, const int32_t *orow, const int32_t *ocol,
-                               const float *wout, const float *lam_new, const float *s_new,
-                               float damping, float *grad_ew, float *grad_t_old,
-                               cudaStream_t s);
+// lam_new: lambda in new ids; s_old: forward scores in original ids.
+cudaError_t LaunchAdjointGrads(const DeviceGraph &g, const float *lam_new, const float *s_old,
+                               float damping, float *grad_ew, float *grad_t_old, cudaStream_t s);
 cudaError_t LaunchL1Norm(const float *x, int64_t n, double *out, cudaStream_t s);
 cudaError_t LaunchGatherOut(const DeviceGraph &g, const float *src_new, float *dst_old,
                             int ncols, cudaStream_t s);

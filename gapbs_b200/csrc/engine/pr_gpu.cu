@@ -20,6 +20,7 @@
 #include "internal.h"
 #include "batched.h"
 #include "blocked.h"
+#include "resident.h"
 
 using prgpu::DeviceGraph;
 using prgpu::Scratch;
@@ -60,6 +61,11 @@ struct pr_gpu {
   // CSR of the last pr_gpu_generate (original ids), kept for download
   int32_t *gen_off = nullptr, *gen_nbr = nullptr;
   int64_t gen_n = 0, gen_m = 0;
+  // resident solves: barrier state, and the page-locked block they report in
+  // (ResidentResult, then kHostTrace doubles of trace)
+  static constexpr int kHostTrace = 4096;
+  prgpu::ResidentCtl *rctl = nullptr;
+  prgpu::ResidentResult *rres = nullptr;
   prgpu::CcScratch cc;    // connected-components work arrays
   prgpu::BfsScratch bfs;  // breadth-first-search work arrays
 };
@@ -266,7 +272,7 @@ cudaError_t Grow(T **p, int64_t *cap, int64_t need) {
 
 void FreeScratch(Scratch *sc) {
   void *ptrs[] = {sc->score, sc->contrib[0], sc->contrib[1], sc->base, sc->outbuf, sc->tele,
-                  sc->aux[0], sc->aux[1], sc->edge_buf, sc->norm,
+                  sc->aux, sc->edge_buf, sc->norm,
                   sc->part1, sc->part2, sc->tick1, sc->trace, sc->ctl};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -279,13 +285,13 @@ int EnsureScratch(pr_gpu_t *h, int64_t n, int ncols, int64_t nblocks, int iters)
   const int64_t cells = n * ncols;
   if (!s.score || s.cap_n < cells) {
     for (float **p : {&s.score, &s.contrib[0], &s.contrib[1], &s.base, &s.outbuf, &s.tele,
-                      &s.aux[0], &s.aux[1]}) {
+                      &s.aux}) {
       if (*p) cudaFree(*p);
       *p = nullptr;
     }
     s.cap_n = 0;
     for (float **p : {&s.score, &s.contrib[0], &s.contrib[1], &s.base, &s.outbuf, &s.tele,
-                      &s.aux[0], &s.aux[1]})
+                      &s.aux})
       PR_CHECK(h, cudaMalloc(p, sizeof(float) * std::max<int64_t>(cells, 1)));
     s.cap_n = cells;
   }
@@ -329,9 +335,10 @@ int EnsureSliceBlocks(pr_gpu_t *h) {
   h->sb_built = true;
   h->loop_blocked.Reset();
   std::string msg;
-  // below about 48 M edges the gather sweep's contribs stay in L1 and L2
-  // (measured: g20, 31 M edges, 0.117 against 0.125 ms per sweep; g21,
-  // 64 M edges, 0.200 against 0.157)
+  // below about 48 M edges a resident gather solve is faster (Kronecker 2^20,
+  // 31 M edges: 0.54 ms a solve against 1.0; 2^21, 64 M edges: 0.95 against
+  // 1.09; 3 M vertices, 76 M edges: 1.42 / 1.47; 2^22, 128 M edges: 1.96 /
+  // 1.67 -- the sizes between keep the layout, as documented in pr_gpu.h)
   if (h->sweep_layout == PR_GPU_SWEEP_AUTO && h->g.m < kAutoBlockedMinEdges) return PR_GPU_OK;
   const int64_t max_pairs = h->sweep_layout == PR_GPU_SWEEP_AUTO
                                 ? h->g.m / 2
@@ -353,6 +360,124 @@ void DropGraph(pr_gpu_t *h) {
   prgpu::FreeDeviceGraph(&h->g);
 }
 
+// Whether a single-column gather solve runs as one resident launch.  It does
+// unless the contribs outgrow what L2 serves well (over 2^23 vertices: 32 MB)
+// and few entries come from the shared-memory tile: then nearly every gather
+// waits on L2 or HBM, and the sweep kernel's larger number of resident warps
+// hides that better (uniform graphs, degree 32, ms a solve, resident against
+// sweep launches: 2^22 vertices 3.4 / 3.7, 2^24 17.5 / 15.5; Kronecker 2^23
+// 4.3 / 6.1).  The adjoint of a directed graph, whose out-rows have no
+// order by length, always does.
+bool UseResident(const pr_gpu_t *h, int kind) {
+  const DeviceGraph &g = h->g;
+  if (kind == prgpu::kKindAdjoint && g.directed) return true;
+  return g.n <= (int64_t(1) << 23) || g.tile_entries >= g.m / 10;
+}
+
+// Single-column gather solve (kind: kKindPlain, kKindPPR or kKindAdjoint) as
+// one launch; in_old / out_old: device buffers in original ids.
+int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float damping,
+                  const float *in_old, float *out_old, int32_t *sweeps_out, double *err_trace) {
+  DeviceGraph &g = h->g;
+  cudaStream_t s = h->stream;
+  const bool out_rows = kind == prgpu::kKindAdjoint && g.directed;
+  prgpu::RowTasks &rt = out_rows ? g.out_tasks : g.in_tasks;
+  if (!rt.ready)
+    PR_CHECK(h, prgpu::BuildRowTasks(static_cast<int32_t>(g.n), out_rows ? g.orowoff : g.rowoff,
+                                     !out_rows, prgpu::ClassesFor(g.m, g.weighted), &rt, s));
+  int sms = 0;
+  PR_CHECK(h, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+  const void *fn = prgpu::ResidentKernel(kind, g.weighted, g.directed);
+  prgpu::ResidentArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.tile = static_cast<int32_t>(std::min<int64_t>(g.n, prgpu::kResidentTile) & ~int64_t(3));
+  int grid = static_cast<int>(
+      std::max<int64_t>(1, std::min<int64_t>(sms, g.m / prgpu::kResidentEntriesPerCta)));
+  int rc = EnsureScratch(h, g.n, 1, 2 * grid, max_iters);
+  if (rc) return rc;
+  Scratch &sc = h->sc;
+  if (!h->rctl) {
+    PR_CHECK(h, cudaMalloc(&h->rctl, sizeof(prgpu::ResidentCtl)));
+    PR_CHECK(h, cudaMemsetAsync(h->rctl, 0, sizeof(prgpu::ResidentCtl), s));
+  }
+  if (!h->rres)
+    PR_CHECK(h, cudaHostAlloc(reinterpret_cast<void **>(&h->rres),
+                              sizeof(prgpu::ResidentResult) + sizeof(double) * pr_gpu::kHostTrace,
+                              cudaHostAllocMapped | cudaHostAllocPortable));
+  double *host_trace = reinterpret_cast<double *>(h->rres + 1);
+  const bool trace_on_host = max_iters <= pr_gpu::kHostTrace;
+  std::memset(h->rres, 0, sizeof(*h->rres));
+  const float n_f = static_cast<float>(g.n);
+  a.n = static_cast<int32_t>(g.n);
+  a.max_iters = max_iters;
+  a.rowoff = out_rows ? g.orowoff : g.rowoff;
+  a.col = out_rows ? g.ocol : g.col;
+  a.win = !g.weighted ? nullptr : (kind == prgpu::kKindAdjoint ? g.wout : g.win);
+  a.odeg = g.odeg;
+  a.rsum = g.rsum;
+  a.perm = g.perm;
+  a.inv = g.inv;
+  a.in_old = in_old;
+  a.out_old = out_old;
+  a.init_scalar = 1.0f / n_f;              // src/pr_spmv.cc:37
+  a.base_scalar = (1.0f - damping) / n_f;  // src/pr_spmv.cc:38
+  a.damping = damping;
+  a.one_minus_d = 1.0f - damping;
+  a.score = sc.score;
+  a.c0 = sc.contrib[0];
+  a.c1 = sc.contrib[1];
+  a.base = sc.base;
+  std::memcpy(a.row_start, rt.row_start, sizeof(a.row_start));
+  std::memcpy(a.task_start, rt.task_start, sizeof(a.task_start));
+  a.segment = rt.segment;
+  a.order = rt.order;
+  a.seg = rt.seg;
+  a.seg_partial = rt.seg_partial;
+  a.ticket = rt.ticket;
+  // a directed graph's rows without entries are still gathered: both contrib
+  // buffers must hold their values
+  a.zero_final_sweep = g.directed ? 2 : 1;
+  a.epsilon = epsilon;
+  a.part = sc.part1;
+  a.trace = trace_on_host ? host_trace : sc.trace;
+  a.ctl = h->rctl;
+  a.res = h->rres;
+  const size_t smem = sizeof(float) * (a.tile + 4);  // and the zero slot
+  PR_CHECK(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(smem)));
+  PR_CHECK(h, cudaEventRecord(h->ev[0], s));
+  void *params[] = {&a};
+  cudaError_t le = cudaSuccess;
+  for (;; grid /= 2) {
+    le = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(prgpu::kResidentThreads), params, smem, s);
+    // a stream that may use part of the GPU only: any grid size solves
+    if (le != cudaErrorCooperativeLaunchTooLarge || grid == 1) break;
+    cudaGetLastError();
+  }
+  PR_CHECK(h, le);
+  PR_CHECK(h, cudaEventRecord(h->ev[3], s));
+  PR_CHECK(h, cudaStreamSynchronize(s));
+  if (h->rres->failed) {
+    PR_CHECK(h, cudaMemsetAsync(h->rctl, 0, sizeof(prgpu::ResidentCtl), s));
+    return SetErr(h, PR_GPU_ECUDA, "a grid barrier of the solve ran out of its wait");
+  }
+  const int sweeps = h->rres->sweeps;
+  if (err_trace) {
+    if (sweeps && trace_on_host) std::memcpy(err_trace, host_trace, sizeof(double) * sweeps);
+    else if (sweeps)
+      PR_CHECK(h, cudaMemcpy(err_trace, sc.trace, sizeof(double) * sweeps, cudaMemcpyDeviceToHost));
+    std::fill(err_trace + sweeps, err_trace + max_iters, 0.0);
+  }
+  if (sweeps_out) *sweeps_out = sweeps;
+  float ms_total = 0;
+  cudaEventElapsedTime(&ms_total, h->ev[0], h->ev[3]);
+  h->last_sweep_ms = h->rres->sweep_ns * 1e-6;
+  h->last_total_ms = ms_total;
+  h->last_launches = 1;
+  h->last_blocked = false;
+  return PR_GPU_OK;
+}
+
 bool UseBlocked(const pr_gpu_t *h) {
   return h->sweep_layout != PR_GPU_SWEEP_GATHER && h->sb.ready && !h->g.weighted;
 }
@@ -370,6 +495,10 @@ int SolveSingle(pr_gpu_t *h, int max_iters, double epsilon, float damping,
                   "the slice-blocked sweep does not fit this graph (weighted, no edges, or more "
                   "source slices than a bin holds)");
   const bool blocked = UseBlocked(h);
+  const int kind = tele_old ? prgpu::kKindPPR : prgpu::kKindPlain;
+  if (!blocked && !h->time_kernels && UseResident(h, kind))
+    return SolveResident(h, kind, max_iters, epsilon, damping, tele_old, out_old, sweeps_out,
+                         err_trace);
   int32_t task_start[prgpu::kNumBins + 1];
   prgpu::PullTasks(g, task_start);
   prgpu::PullArgs probe;
@@ -556,14 +685,28 @@ int SolveSingle(pr_gpu_t *h, int max_iters, double epsilon, float damping,
 int SolveAdjoint(pr_gpu_t *h, int max_iters, double epsilon, float damping, const float *w_old,
                  const float *s_old, float *grad_t_old, float *grad_ew) {
   DeviceGraph &g = h->g;
+  if (UseResident(h, prgpu::kKindAdjoint)) {
+    int rc = SolveResident(h, prgpu::kKindAdjoint, max_iters, epsilon, damping, w_old, grad_t_old,
+                           &h->last_adjoint_sweeps, nullptr);
+    if (rc) return rc;
+    PR_CHECK(h, prgpu::LaunchAdjointGrads(g, h->sc.score, s_old, damping, grad_ew, nullptr,
+                                          h->stream));
+    PR_CHECK(h, cudaEventRecord(h->ev[3], h->stream));
+    PR_CHECK(h, cudaStreamSynchronize(h->stream));
+    float ms_total = 0;
+    cudaEventElapsedTime(&ms_total, h->ev[0], h->ev[3]);
+    h->last_total_ms = ms_total;
+    if (grad_ew) h->last_launches++;
+    return PR_GPU_OK;
+  }
+  // undirected graphs only (UseResident)
   int32_t task_start[prgpu::kNumBins + 1];
   prgpu::PullTasks(g, task_start);
-  const bool generic = g.directed;
   prgpu::PullArgs probe;
   std::memset(&probe, 0, sizeof(probe));
   probe.kind = prgpu::kKindAdjoint;
   probe.win = g.weighted ? g.wout : nullptr;
-  const void *adj_fn = generic ? prgpu::PullGenericKernel(probe) : prgpu::PullSweepKernel(probe);
+  const void *adj_fn = prgpu::PullSweepKernel(probe);
   const int nblocks = prgpu::PullGrid(adj_fn);
   int rc = EnsureScratch(h, g.n, 1, nblocks, max_iters);
   if (rc) return rc;
@@ -571,42 +714,37 @@ int SolveAdjoint(pr_gpu_t *h, int max_iters, double epsilon, float damping, cons
   cudaStream_t s = h->stream;
   int64_t launches = 0;
   PR_CHECK(h, cudaEventRecord(h->ev[0], s));
-  // w and s in new ids; lambda_0 = w
+  // w in new ids; lambda_0 = w
   PR_CHECK(h, prgpu::LaunchScatterIn(g, w_old, sc.base, 1, s));
-  PR_CHECK(h, prgpu::LaunchScatterIn(g, s_old, sc.aux[0], 1, s));
   PR_CHECK(h, prgpu::LaunchL1Norm(w_old, g.n, sc.norm, s));
-  launches += 3;
+  launches += 2;
   PR_CHECK(h, cudaMemcpyAsync(sc.score, sc.base, sizeof(float) * g.n, cudaMemcpyDeviceToDevice, s));
   PR_CHECK(h, cudaMemcpyAsync(sc.contrib[0], sc.base, sizeof(float) * g.n, cudaMemcpyDeviceToDevice, s));
   double wnorm = 0;
   PR_CHECK(h, cudaMemcpyAsync(&wnorm, sc.norm, sizeof(double), cudaMemcpyDeviceToHost, s));
   PR_CHECK(h, cudaStreamSynchronize(s));
   PR_CHECK(h, prgpu::LaunchResetCtl(sc, nblocks, max_iters, s));
-  const int32_t *orow = generic ? g.orowoff : g.rowoff;
-  const int32_t *ocol = generic ? g.ocol : g.col;
   prgpu::PullArgs a;
   std::memset(&a, 0, sizeof(a));
   a.n = static_cast<int32_t>(g.n);
   a.kind = prgpu::kKindAdjoint;
-  a.rowoff = orow;
-  a.col = ocol;
+  a.rowoff = g.rowoff;
+  a.col = g.col;
   a.win = g.weighted ? g.wout : nullptr;
   a.odeg = nullptr;
   a.rsum = g.weighted ? g.rsum : nullptr;
   a.base_vec = sc.base;
   a.damping = damping;
   a.score = sc.score;
-  if (!generic) {
-    for (int b = 0; b <= prgpu::kNumBins; b++) {
-      a.task_start[b] = task_start[b];
-      a.bin_row[b] = static_cast<int32_t>(g.bin_row_start[b]);
-    }
-    a.nseg = static_cast<int32_t>(g.num_segments);
-    a.seg_row = g.seg_row;
-    a.seg_first = g.seg_first;
-    a.hub_ticket = g.hub_ticket;
-    a.seg_partial = g.seg_partial;
+  for (int b = 0; b <= prgpu::kNumBins; b++) {
+    a.task_start[b] = task_start[b];
+    a.bin_row[b] = static_cast<int32_t>(g.bin_row_start[b]);
   }
+  a.nseg = static_cast<int32_t>(g.num_segments);
+  a.seg_row = g.seg_row;
+  a.seg_first = g.seg_first;
+  a.hub_ticket = g.hub_ticket;
+  a.seg_partial = g.seg_partial;
   a.part1 = sc.part1;
   a.part2 = sc.part2;
   a.tick1 = sc.tick1;
@@ -623,8 +761,7 @@ int SolveAdjoint(pr_gpu_t *h, int max_iters, double epsilon, float damping, cons
     PR_CHECK(h, h->loop_adjoint.Launch(adj_fn, dim3(nblocks), dim3(prgpu::kSweepThreads), &a, sizeof(a),
                                        &sc.ctl->loop, max_iters, s));
   PR_CHECK(h, cudaEventRecord(h->ev[2], s));
-  PR_CHECK(h, prgpu::LaunchAdjointGrads(g, orow, ocol, g.weighted ? g.wout : nullptr, sc.score,
-                                        sc.aux[0], damping, grad_ew, grad_t_old, s));
+  PR_CHECK(h, prgpu::LaunchAdjointGrads(g, sc.score, s_old, damping, grad_ew, grad_t_old, s));
   launches += 2;
   PR_CHECK(h, cudaEventRecord(h->ev[3], s));
   prgpu::SweepCtl ctl;
@@ -677,6 +814,8 @@ void pr_gpu_destroy(pr_gpu_t *h) {
     if (h->pinned[i]) cudaFreeHost(h->pinned[i]);
     if (h->pin_ev[i]) cudaEventDestroy(h->pin_ev[i]);
   }
+  if (h->rctl) cudaFree(h->rctl);
+  if (h->rres) cudaFreeHost(h->rres);
   for (auto &e : h->ev)
     if (e) cudaEventDestroy(e);
   for (auto &e : h->kev)
@@ -1064,9 +1203,9 @@ int pr_gpu_adjoint(pr_gpu_t *h, int max_iters, double epsilon, float damping,
   Scratch &sc = h->sc;
   if (grad_edge_w) PR_CHECK(h, Grow(&sc.edge_buf, &sc.cap_edges, std::max<int64_t>(m, 1)));
   rc = CopyToDevice(h, sc.tele, loss_w, sizeof(float) * n);
-  if (!rc) rc = CopyToDevice(h, sc.aux[1], scores, sizeof(float) * n);
+  if (!rc) rc = CopyToDevice(h, sc.aux, scores, sizeof(float) * n);
   if (rc) return rc;
-  rc = pr_gpu_adjoint_device(h, max_iters, epsilon, damping, sc.tele, sc.aux[1],
+  rc = pr_gpu_adjoint_device(h, max_iters, epsilon, damping, sc.tele, sc.aux,
                              grad_teleport ? sc.outbuf : nullptr,
                              grad_edge_w ? sc.edge_buf : nullptr, sweeps_out);
   if (rc) return rc;

@@ -226,6 +226,8 @@ void FreeDeviceGraph(DeviceGraph *g) {
                   g->seg_partial};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  FreeRowTasks(&g->in_tasks);
+  FreeRowTasks(&g->out_tasks);
   BinConfig keep = g->bins;
   *g = DeviceGraph();
   g->bins = keep;
@@ -370,7 +372,12 @@ cudaError_t BuildDeviceGraph(DeviceGraph *g, int64_t n, int64_t m,
   bin_bounds_kernel<<<1, 32, 0, s>>>(n, deg_sorted, g->bins, d_bins);
   PR_TRY(cudaMemcpyAsync(g->bin_row_start, d_bins, sizeof(int64_t) * (kNumBins + 1),
                          cudaMemcpyDeviceToHost, s));
+  int32_t tile_entries = static_cast<int32_t>(m);
+  if (n > kResidentTile)
+    PR_TRY(cudaMemcpyAsync(&tile_entries, g->rowoff + kResidentTile, sizeof(int32_t),
+                           cudaMemcpyDeviceToHost, s));
   PR_TRY(cudaStreamSynchronize(s));
+  g->tile_entries = tile_entries;
   if (flag) {
     *err = "invalid CSR:" + FlagText(flag);
     cleanup();

@@ -288,41 +288,6 @@ pull_sweep_kernel(const PullArgs a) {
   grid_finish(a, it, block_err, sred);
 }
 
-// ---- generic warp-per-row sweep (unsorted CSR, grid-stride) ----------------
-
-template <bool W, int KIND>
-__global__ void __launch_bounds__(kSweepThreads)
-pull_generic_kernel(const PullArgs a) {
-  if (*reinterpret_cast<volatile const int *>(&a.ctl->loop.done)) return;
-  const int it = *reinterpret_cast<volatile const int *>(&a.ctl->loop.loops);
-  const float *cin = (it & 1) ? a.c1 : a.c0;
-  float *cout = (it & 1) ? a.c0 : a.c1;
-  __shared__ double sred[kSweepThreads / 32];
-  const uint64_t ps = policy_evict_first();
-  const uint64_t pg = policy_evict_last();
-  const int lane = threadIdx.x & 31;
-  const int warps = a.nblocks * (kSweepThreads / 32);
-  double err = 0.0;
-  for (int u = blockIdx.x * (kSweepThreads / 32) + (threadIdx.x >> 5); u < a.n; u += warps) {
-    const int s = a.rowoff[u], e = a.rowoff[u + 1];
-    float acc = lane_partial<32, W>(a, cin, s, e, lane, ps, pg);
-    acc = group_sum<32>(acc);
-    if (lane == 0)
-      err += finish_row<W, false, KIND>(a, cout, u, s, e, acc, ld_score(a.score + u, ps), ps, pg);
-  }
-  const double block_err = block_sum_d<kSweepThreads>(err, sred);
-  grid_finish(a, it, block_err, sred);
-}
-
-const void *PullGenericKernel(const PullArgs &a) {
-  const bool W = a.win != nullptr;
-  if (a.kind == kKindAdjoint)
-    return W ? reinterpret_cast<const void *>(pull_generic_kernel<true, kKindAdjoint>)
-             : reinterpret_cast<const void *>(pull_generic_kernel<false, kKindAdjoint>);
-  return W ? reinterpret_cast<const void *>(pull_generic_kernel<true, kKindPPR>)
-           : reinterpret_cast<const void *>(pull_generic_kernel<false, kKindPPR>);
-}
-
 // ---- adjoint gradients ---------------------------------------------------------
 
 // One warp per renumbered out-row v:
@@ -335,7 +300,7 @@ __global__ void adjoint_edge_grad_kernel(int32_t n, const int32_t *__restrict__ 
                                          const int32_t *__restrict__ perm,
                                          const int32_t *__restrict__ orig_off,
                                          const float *__restrict__ lam,
-                                         const float *__restrict__ sv, float damping,
+                                         const float *__restrict__ s_old, float damping,
                                          float *grad_ew) {
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -350,8 +315,9 @@ __global__ void adjoint_edge_grad_kernel(int32_t n, const int32_t *__restrict__ 
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   const double S = rsum ? static_cast<double>(rsum[v]) : static_cast<double>(e - s);
   const double plam = acc / S;
-  const double coef = static_cast<double>(damping) * sv[v] / S;
-  const int64_t base = orig_off[perm[v]];
+  const int pv = perm[v];
+  const double coef = static_cast<double>(damping) * s_old[pv] / S;
+  const int64_t base = orig_off[pv];
   for (int j = s + lane; j < e; j += 32)
     grad_ew[base + (j - s)] = static_cast<float>(coef * (lam[ocol[j]] - plam));
 }
@@ -364,15 +330,15 @@ __global__ void adjoint_teleport_grad_kernel(int32_t n, const int32_t *__restric
   grad_t[v] = __fmul_rn(omd, lam[inv[v]]);
 }
 
-cudaError_t LaunchAdjointGrads(const DeviceGraph &g, const int32_t *orow, const int32_t *ocol,
-                               const float *wout, const float *lam_new, const float *s_new,
-                               float damping, float *grad_ew, float *grad_t_old,
-                               cudaStream_t s) {
+cudaError_t LaunchAdjointGrads(const DeviceGraph &g, const float *lam_new, const float *s_old,
+                               float damping, float *grad_ew, float *grad_t_old, cudaStream_t s) {
   const int n = static_cast<int>(g.n);
+  const int32_t *orow = g.directed ? g.orowoff : g.rowoff;
+  const int32_t *ocol = g.directed ? g.ocol : g.col;
   if (grad_ew) {
     adjoint_edge_grad_kernel<<<static_cast<unsigned>((static_cast<int64_t>(n) * 32 + 255) / 256), 256, 0, s>>>(
-        n, orow, ocol, wout, g.weighted ? g.rsum : nullptr, g.perm, g.orig_out_off, lam_new, s_new,
-        damping, grad_ew);
+        n, orow, ocol, g.weighted ? g.wout : nullptr, g.weighted ? g.rsum : nullptr, g.perm,
+        g.orig_out_off, lam_new, s_old, damping, grad_ew);
   }
   if (grad_t_old)
     adjoint_teleport_grad_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, g.inv, lam_new, 1.0f - damping,
