@@ -16,9 +16,9 @@
 // gather, so a sector is skipped once its eight columns have retired.
 //
 // Work split (rows renumbered by descending in-degree, as for the plain
-// sweep): a persistent grid (SMs x resident blocks) first takes the hub-row
-// segments block-cooperatively (the row's last segment block sums the
-// segment partials in segment order), then every warp takes whole rows,
+// sweep): a persistent grid (SMs x resident blocks) first takes the segments
+// of the long rows, a warp each (at the end of the sweep the warp that brings
+// a row's last segment adds the partials), then every warp takes whole rows,
 // interleaved across the grid, and finally the short rows (fewer in-entries
 // than two rounds of a warp's gathers) go one row per lane group, 32/L rows
 // per warp at once, so the per-row work (offsets, old score, update, stores)
@@ -42,6 +42,7 @@
 
 #include "batched.h"
 #include "common.cuh"
+#include "resident.h"
 
 namespace prgpu {
 
@@ -50,6 +51,9 @@ namespace {
 constexpr int kBT = 256;       // threads per block
 constexpr int kBW = kBT / 32;  // warps per block
 constexpr int kUnroll = 4;     // gather instructions in flight per lane
+// Blocks whose column partials one block adds up: about the square root of
+// the grid (148 x 8), so that neither stage of the reduction is long.
+constexpr int kColGroup = 32;
 constexpr int64_t kL1GatherBytes = 96 * 1024;  // L1 budget for hub rows per SM
 
 struct BatchArgs {
@@ -67,11 +71,11 @@ struct BatchArgs {
   float *C0;  // contrib ping-pong: sweep k gathers C[k & 1], writes C[(k + 1) & 1]
   float *C1;
   int32_t nseg;
-  int32_t hub_rows;
+  int32_t segment;    // entries of a long row's segment
+  int32_t long_rows;  // rows cut into segments
   int32_t zero_start;
-  const int32_t *__restrict__ seg_row;
-  const int32_t *__restrict__ seg_first;
-  unsigned *hub_ticket;
+  const int4 *__restrict__ seg;
+  unsigned *ticket;
   float *seg_partial;
   double *part1;
   double *part2;
@@ -118,25 +122,30 @@ __device__ __forceinline__ float4 gather_row4(const BatchArgs &a, const float *C
 // Sum over entries [s, e) of w_e * Cin[v_e, 4*gl .. 4*gl+3], where lane group
 // grp = lane / L takes every (32/L)-th entry; the caller reduces across
 // groups.  Indices (and weights) are loaded 32 at a time and broadcast.
-template <int L, bool W>
+// FIRST: the sweep from s_0 = t.  Only rows with a nonzero teleport entry
+// (tflag) have a contrib; the others, which the init leaves unwritten, are
+// zero and not gathered.
+template <int L, bool W, bool FIRST>
 __device__ __forceinline__ float4 row_accumulate(const BatchArgs &a, const float *Cin, int s, int e,
-                                                 int lane, bool gather, uint64_t ps, uint64_t pg,
-                                                 bool have_first = false, int idx_first = 0,
-                                                 float w_first = 0.f) {
+                                                 int lane, bool gather, uint64_t ps, uint64_t pg) {
   constexpr int NPW = 32 / L;
   const int grp = lane / L, gl = lane % L;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  int idx_next = 0;
+  float w_next = 0.f;
+  if (s + lane < e) {
+    idx_next = ld_stream_s32(a.col + s + lane, ps);
+    if (W) w_next = ld_stream_f32(a.win + s + lane, ps);
+  }
   for (int j0 = s; j0 < e; j0 += 32) {
     const int cnt = min(32, e - j0);
-    int idx = 0;
-    float w = 0.f;
-    if (have_first && j0 == s) {
-      idx = idx_first;
-      w = w_first;
-    } else if (lane < cnt) {
-      idx = ld_stream_s32(a.col + j0 + lane, ps);
-      if (W) w = ld_stream_f32(a.win + j0 + lane, ps);
+    int idx = idx_next;
+    const float w = w_next;
+    if (j0 + 32 + lane < e) {  // fetched while this round's rows are gathered
+      idx_next = ld_stream_s32(a.col + j0 + 32 + lane, ps);
+      if (W) w_next = ld_stream_f32(a.win + j0 + 32 + lane, ps);
     }
+    if (FIRST && lane < cnt && !__ldg(a.tflag + idx)) idx = -1;
     for (int k = 0; k < cnt; k += NPW * kUnroll) {
       float4 x[kUnroll];
       float wk[kUnroll];
@@ -146,7 +155,7 @@ __device__ __forceinline__ float4 row_accumulate(const BatchArgs &a, const float
         const int v = __shfl_sync(0xffffffffu, idx, kk & 31);
         wk[q] = W ? __shfl_sync(0xffffffffu, w, kk & 31) : 1.f;
         x[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gather && kk < cnt) x[q] = gather_row4<L>(a, Cin, v, gl, pg);
+        if (gather && kk < cnt && (!FIRST || v >= 0)) x[q] = gather_row4<L>(a, Cin, v, gl, pg);
       }
 #pragma unroll
       for (int q = 0; q < kUnroll; q++) {
@@ -177,7 +186,7 @@ __device__ __forceinline__ float4 row_accumulate(const BatchArgs &a, const float
 // over it, kUnroll gathers in flight per group.  Each lane loads CH / L of
 // every CH consecutive indices of its group's row; the loop runs to the
 // longest row of the warp (warp-uniform trip count, shuffles stay converged).
-template <int L, bool W>
+template <int L, bool W, bool FIRST>
 __device__ __forceinline__ float4 group_accumulate(const BatchArgs &a, const float *Cin, int s,
                                                    int len, int lane, bool gather, uint64_t ps,
                                                    uint64_t pg) {
@@ -199,6 +208,7 @@ __device__ __forceinline__ float4 group_accumulate(const BatchArgs &a, const flo
       if (j < len) {
         idx[r] = ld_stream_s32(a.col + s + j, ps);
         if (W) w[r] = ld_stream_f32(a.win + s + j, ps);
+        if (FIRST && !__ldg(a.tflag + idx[r])) idx[r] = -1;
       }
     }
 #pragma unroll
@@ -213,7 +223,8 @@ __device__ __forceinline__ float4 group_accumulate(const BatchArgs &a, const flo
           const int v = __shfl_sync(0xffffffffu, idx[kk / L], srcl);
           wk[q] = W ? __shfl_sync(0xffffffffu, w[kk / L], srcl) : 1.f;
           x[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (gather && j0 + kk < len) x[q] = gather_row4<L>(a, Cin, v, gl, pg);
+          if (gather && j0 + kk < len && (!FIRST || v >= 0))
+            x[q] = gather_row4<L>(a, Cin, v, gl, pg);
         }
 #pragma unroll
         for (int q = 0; q < kUnroll; q++) {
@@ -234,6 +245,23 @@ __device__ __forceinline__ float4 group_accumulate(const BatchArgs &a, const flo
 
 __device__ __forceinline__ float comp(const float4 &v, int c) {
   return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w;
+}
+
+// Column sums of a count x Bp block of partials, in a fixed order: thread
+// r Bp + c adds rows r, r + kBT / Bp, ... of column c, thread c the kBT / Bp
+// results.  Valid in threads below Bp; buf: kBT doubles.  (One thread a column
+// added up to 512 rows one load after the other: 80 us a sweep.)
+__device__ __forceinline__ double column_sums(const double *part, int count, int Bp, double *buf) {
+  const int c = threadIdx.x & (Bp - 1), r0 = threadIdx.x / Bp, nr = kBT / Bp;
+  double v = 0;
+  for (int r = r0; r < count; r += nr) v += __ldcg(part + static_cast<int64_t>(r) * Bp + c);
+  __syncthreads();  // buf may still be read
+  buf[threadIdx.x] = v;
+  __syncthreads();
+  double sum = 0;
+  if (threadIdx.x < Bp)
+    for (int r = 0; r < nr; r++) sum += buf[r * Bp + threadIdx.x];
+  return sum;
 }
 
 // Updates the four columns 4*gl.. of row u from their sums (active columns
@@ -258,102 +286,45 @@ __device__ __forceinline__ void finish4(const BatchArgs &a, float *Cout, int u, 
   st_hint_v4(reinterpret_cast<float4 *>(Cout + i), make_float4(cv[0], cv[1], cv[2], cv[3]), pl);
 }
 
-template <int L, bool W, bool DIR>
-__global__ void __launch_bounds__(kBT, W ? 6 : 8) batch_sweep_kernel(const BatchArgs a) {
-  if (*reinterpret_cast<volatile const int *>(&a.ctl->loop.done)) return;
-  const int it = *reinterpret_cast<volatile const int *>(&a.ctl->loop.loops);
-  const float *Cin = (it & 1) ? a.C1 : a.C0;
-  float *Cout = (it & 1) ? a.C0 : a.C1;
-  __shared__ double serr[kBW][kMaxTile];
-  __shared__ double scol[kMaxTile];
-  __shared__ float sacc[kBW][kMaxTile];
-  __shared__ int s_last;
-  const uint64_t ps = policy_evict_first();
-  const uint64_t pg = policy_evict_last();
+// All rows of one sweep.
+template <int L, bool W, bool DIR, bool FIRST>
+__device__ __forceinline__ void sweep_rows(const BatchArgs &a, int it, const float *Cin,
+                                           float *Cout, unsigned long long active, double *err,
+                                           uint64_t ps, uint64_t pg) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int gl = lane % L;
   const int Bp = a.Bp;
-  const unsigned long long active =
-      *reinterpret_cast<volatile const unsigned long long *>(&a.ctl->active);
   const unsigned active4 = static_cast<unsigned>((active >> (4 * gl)) & 0xFull);
   const bool gather = active4 != 0u;
-  // per-thread FP64 error of its four columns, in shared memory (column c of
-  // thread t at s_err[c][t]) to keep registers for gathers in flight
-  __shared__ double s_err[4][kBT];
-  double *err = &s_err[0][threadIdx.x];
-#pragma unroll
-  for (int c = 0; c < 4; c++) err[c * kBT] = 0.0;
-  if (threadIdx.x < kMaxTile) scol[threadIdx.x] = 0;
 
-  // ---- hub segments, block-cooperative
-  for (int seg = blockIdx.x; seg < a.nseg; seg += gridDim.x) {
-    const int u = a.seg_row[seg];
-    const int first = a.seg_first[u];
-    const int nseg = a.seg_first[u + 1] - first;
-    const int rs = a.rowoff[u], re = a.rowoff[u + 1];
-    const int s = rs + (seg - first) * kSegEntries;
-    const int e = min(re, s + kSegEntries);
-    const int per = (e - s + kBW - 1) / kBW;
-    const int ws = min(e, s + wid * per), we = min(e, ws + per);
-    const float4 acc = row_accumulate<L, W>(a, Cin, ws, we, lane, gather, ps, pg);
-    if (lane < L) {
-      sacc[wid][4 * gl + 0] = acc.x;
-      sacc[wid][4 * gl + 1] = acc.y;
-      sacc[wid][4 * gl + 2] = acc.z;
-      sacc[wid][4 * gl + 3] = acc.w;
-    }
-    __syncthreads();
-    if (threadIdx.x < Bp) {
-      float p = 0.f;
-      for (int w = 0; w < kBW; w++) p += sacc[w][threadIdx.x];
-      a.seg_partial[static_cast<int64_t>(seg) * Bp + threadIdx.x] = p;
-    }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const unsigned t = atomicAdd(a.hub_ticket + u, 1u);
-      s_last = (t == static_cast<unsigned>(nseg - 1));
-    }
-    __syncthreads();
-    if (s_last) {
-      // the row's last segment block finishes the row: thread c owns column c
-      __threadfence();
-      const int c = threadIdx.x;
-      if (c < Bp && ((active >> c) & 1ull)) {
-        float sum = 0.f;
-        for (int k = 0; k < nseg; k++)
-          sum = __fadd_rn(sum, __ldcg(a.seg_partial + static_cast<int64_t>(first + k) * Bp + c));
-        const int64_t i = static_cast<int64_t>(u) * Bp + c;
-        const float old = ld_score(a.S + i, ps);
-        const float b0 = a.tflag[u] ? a.base[i] : 0.f;
-        const float nw = __fadd_rn(b0, __fmul_rn(a.damping, sum));
-        st_hint_f32(a.S + i, nw, ps);
-        st_hint_f32(Cout + i, __fdiv_rn(nw, bdenom<W, DIR>(a, u)), pg);
-        scol[c] += static_cast<double>(fabsf(__fsub_rn(nw, old)));
-      }
-      if (threadIdx.x == 0) a.hub_ticket[u] = 0;
-    }
-    __syncthreads();
+  // ---- segments of the long rows, one warp each; the partials wait in L2
+  // until the end of the sweep
+  const int gw = blockIdx.x * kBW + wid;
+  const int nw = gridDim.x * kBW;
+  for (int k = gw; k < a.nseg; k += nw) {
+    const int4 sg = a.seg[k];  // row, the row's first segment, first entry, end
+    const float4 acc = row_accumulate<L, W, FIRST>(a, Cin, sg.z, sg.w, lane, gather, ps, pg);
+    if (lane < L && gather)
+      *reinterpret_cast<float4 *>(a.seg_partial + static_cast<int64_t>(k) * Bp + 4 * gl) = acc;
   }
 
   // ---- every other row: one warp per row, interleaved across the grid
-  const int gw = blockIdx.x * kBW + wid;
-  const int nw = gridDim.x * kBW;
   // Rows without in-neighbours hold new = base from the first sweep on; their
   // contrib is final once both ping-pong buffers hold it (after the second
   // sweep; an undirected graph never gathers it at all).  Later sweeps skip
   // them: their scores cannot change and their L1 change is exactly zero.
   const int row_end = (it >= a.zero_final_sweep) ? a.zero_start : a.n;
-  const int warp_end = min(max(a.short_start, a.hub_rows), row_end);
-  for (int u = a.hub_rows + gw; u < warp_end; u += nw) {
+  const int warp_end = min(max(a.short_start, a.long_rows), row_end);
+  for (int u = a.long_rows + gw; u < warp_end; u += nw) {
     float4 old = make_float4(0.f, 0.f, 0.f, 0.f), bs = old;
     const int64_t i = static_cast<int64_t>(u) * Bp + 4 * gl;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (u < a.zero_start)
-      acc = row_accumulate<L, W>(a, Cin, a.rowoff[u], a.rowoff[u + 1], lane, gather, ps, pg);
+      acc = row_accumulate<L, W, FIRST>(a, Cin, a.rowoff[u], a.rowoff[u + 1], lane, gather, ps, pg);
     if (lane < L && gather) {
-      old = ld_score_v4(reinterpret_cast<const float4 *>(a.S + i), ps);
-      if (__ldg(a.tflag + u)) bs = ld_stream_v4f(reinterpret_cast<const float4 *>(a.base + i), ps);
+      const bool seeded = __ldg(a.tflag + u) != 0;
+      if (!FIRST || seeded) old = ld_score_v4(reinterpret_cast<const float4 *>(a.S + i), ps);
+      if (seeded) bs = ld_stream_v4f(reinterpret_cast<const float4 *>(a.base + i), ps);
       finish4<W, DIR>(a, Cout, u, gl, active4, acc, old, bs, bdenom<W, DIR>(a, u), err, ps,
                       pg);
     }
@@ -361,7 +332,7 @@ __global__ void __launch_bounds__(kBT, W ? 6 : 8) batch_sweep_kernel(const Batch
   {
     constexpr int NPW = 32 / L;
     const int grp = lane / L;
-    const int sbeg = max(warp_end, a.hub_rows);
+    const int sbeg = max(warp_end, a.long_rows);
     for (int u0 = sbeg + gw * NPW; u0 < row_end; u0 += nw * NPW) {
       const int u = u0 + grp;
       const bool valid = u < row_end;
@@ -372,15 +343,80 @@ __global__ void __launch_bounds__(kBT, W ? 6 : 8) batch_sweep_kernel(const Batch
       }
       float4 old = make_float4(0.f, 0.f, 0.f, 0.f), bs = old;
       const int64_t i = static_cast<int64_t>(u) * Bp + 4 * gl;
-      const float4 acc = group_accumulate<L, W>(a, Cin, s, len, lane, gather, ps, pg);
+      const float4 acc = group_accumulate<L, W, FIRST>(a, Cin, s, len, lane, gather, ps, pg);
       if (valid && gather) {
-        old = ld_score_v4(reinterpret_cast<const float4 *>(a.S + i), ps);
-        if (__ldg(a.tflag + u)) bs = ld_stream_v4f(reinterpret_cast<const float4 *>(a.base + i), ps);
+        const bool seeded = __ldg(a.tflag + u) != 0;
+        if (!FIRST || seeded) old = ld_score_v4(reinterpret_cast<const float4 *>(a.S + i), ps);
+        if (seeded) bs = ld_stream_v4f(reinterpret_cast<const float4 *>(a.base + i), ps);
         finish4<W, DIR>(a, Cout, u, gl, active4, acc, old, bs, bdenom<W, DIR>(a, u), err, ps,
                         pg);
       }
     }
   }
+
+  // ---- long rows: the warp that brings a row's last segment (per-row
+  // ticket) adds the row's partials by a fixed tree and updates the row
+  if (gw < a.nseg) {
+    __threadfence();
+    for (int k = gw; k < a.nseg; k += nw) {
+      const int4 sg = a.seg[k];
+      const int u = sg.x;
+      const int nseg = (a.rowoff[u + 1] - a.rowoff[u] + a.segment - 1) / a.segment;
+      int last = 0;
+      if (lane == 0) last = atomicAdd(a.ticket + sg.y, 1u) == static_cast<unsigned>(nseg - 1);
+      if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+      __threadfence();
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (gather)
+        for (int j = lane / L; j < nseg; j += 32 / L)
+          acc = f4add(acc, __ldcg(reinterpret_cast<const float4 *>(
+                               a.seg_partial + static_cast<int64_t>(sg.y + j) * Bp + 4 * gl)));
+#pragma unroll
+      for (int o = L; o < 32; o <<= 1) {
+        acc.x += __shfl_xor_sync(0xffffffffu, acc.x, o);
+        acc.y += __shfl_xor_sync(0xffffffffu, acc.y, o);
+        acc.z += __shfl_xor_sync(0xffffffffu, acc.z, o);
+        acc.w += __shfl_xor_sync(0xffffffffu, acc.w, o);
+      }
+      if (lane == 0) a.ticket[sg.y] = 0;
+      if (lane < L && gather) {
+        const int64_t i = static_cast<int64_t>(u) * Bp + 4 * gl;
+        const bool seeded = __ldg(a.tflag + u) != 0;
+        float4 old = make_float4(0.f, 0.f, 0.f, 0.f), bs = old;
+        if (!FIRST || seeded) old = ld_score_v4(reinterpret_cast<const float4 *>(a.S + i), ps);
+        if (seeded) bs = ld_stream_v4f(reinterpret_cast<const float4 *>(a.base + i), ps);
+        finish4<W, DIR>(a, Cout, u, gl, active4, acc, old, bs, bdenom<W, DIR>(a, u), err, ps, pg);
+      }
+    }
+  }
+}
+
+template <int L, bool W, bool DIR>
+__global__ void __launch_bounds__(kBT, W ? 6 : 8) batch_sweep_kernel(const BatchArgs a) {
+  if (*reinterpret_cast<volatile const int *>(&a.ctl->loop.done)) return;
+  const int it = *reinterpret_cast<volatile const int *>(&a.ctl->loop.loops);
+  const float *Cin = (it & 1) ? a.C1 : a.C0;
+  float *Cout = (it & 1) ? a.C0 : a.C1;
+  __shared__ double serr[kBW][kMaxTile];
+  __shared__ int s_last;
+  const uint64_t ps = policy_evict_first();
+  const uint64_t pg = policy_evict_last();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int gl = lane % L;
+  const int Bp = a.Bp;
+  const unsigned long long active =
+      *reinterpret_cast<volatile const unsigned long long *>(&a.ctl->active);
+  // per-thread FP64 error of its four columns, in shared memory (column c of
+  // thread t at s_err[c][t]) to keep registers for gathers in flight
+  __shared__ double s_err[4][kBT];
+  double *err = &s_err[0][threadIdx.x];
+#pragma unroll
+  for (int c = 0; c < 4; c++) err[c * kBT] = 0.0;
+
+  if (it == 0)
+    sweep_rows<L, W, DIR, true>(a, it, Cin, Cout, active, err, ps, pg);
+  else
+    sweep_rows<L, W, DIR, false>(a, it, Cin, Cout, active, err, ps, pg);
   // lane groups hold partial errors of the same columns: combine them
   double errc[4];
 #pragma unroll
@@ -398,15 +434,15 @@ __global__ void __launch_bounds__(kBT, W ? 6 : 8) batch_sweep_kernel(const Batch
   __syncthreads();
   const int b = blockIdx.x;
   if (threadIdx.x < Bp) {
-    double p = scol[threadIdx.x];
+    double p = 0;
     for (int w = 0; w < kBW; w++) p += serr[w][threadIdx.x];
     a.part1[static_cast<int64_t>(b) * Bp + threadIdx.x] = p;
   }
   __threadfence();
   __syncthreads();
-  const int g = b / kReduceGroup;
-  const int gsize = min(kReduceGroup, a.nblocks - g * kReduceGroup);
-  const int ngroups = (a.nblocks + kReduceGroup - 1) / kReduceGroup;
+  const int g = b / kColGroup;
+  const int gsize = min(kColGroup, a.nblocks - g * kColGroup);
+  const int ngroups = (a.nblocks + kColGroup - 1) / kColGroup;
   if (threadIdx.x == 0) {
     const unsigned t = atomicAdd(a.tick1 + g, 1u);
     s_last = (t == static_cast<unsigned>(gsize - 1));
@@ -414,12 +450,8 @@ __global__ void __launch_bounds__(kBT, W ? 6 : 8) batch_sweep_kernel(const Batch
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  if (threadIdx.x < Bp) {
-    double p = 0;
-    for (int i = 0; i < gsize; i++)
-      p += __ldcg(a.part1 + static_cast<int64_t>(g * kReduceGroup + i) * Bp + threadIdx.x);
-    a.part2[static_cast<int64_t>(g) * Bp + threadIdx.x] = p;
-  }
+  double tot = column_sums(a.part1 + static_cast<int64_t>(g) * kColGroup * Bp, gsize, Bp, s_err[0]);
+  if (threadIdx.x < Bp) a.part2[static_cast<int64_t>(g) * Bp + threadIdx.x] = tot;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -430,13 +462,11 @@ __global__ void __launch_bounds__(kBT, W ? 6 : 8) batch_sweep_kernel(const Batch
   __syncthreads();
   if (!s_last) return;
   __threadfence();
+  tot = column_sums(a.part2, ngroups, Bp, s_err[0]);
   __shared__ unsigned long long s_retire;
   if (threadIdx.x == 0) s_retire = 0ull;
   __syncthreads();
   if (threadIdx.x < Bp && ((active >> threadIdx.x) & 1ull)) {
-    double tot = 0;
-    for (int i = 0; i < ngroups; i++)
-      tot += __ldcg(a.part2 + static_cast<int64_t>(i) * Bp + threadIdx.x);
     a.trace[static_cast<int64_t>(it) * Bp + threadIdx.x] = tot;
     a.sweeps[threadIdx.x] = it + 1;
     if (tot < a.epsilon) atomicOr(&s_retire, 1ull << threadIdx.x);
@@ -514,8 +544,9 @@ __global__ void __launch_bounds__(kCopyThreads)
 }
 
 // Tile init, one thread per four columns of a row: S = t, C = t / S_v,
-// base = (1-d) t (written only on rows with a nonzero teleport entry, which
-// tflag marks); padding columns are zero.  Cell i is row u = i >> lq,
+// base = (1-d) t, written only on rows with a nonzero teleport entry, which
+// tflag marks: the first sweep takes the others as zero and writes them (S
+// on all rows when no sweep will run); padding columns are zero.  Cell i is row u = i >> lq,
 // columns 4 * (i & (Bp/4 - 1)) ..; a row's cells are consecutive lanes of
 // one warp (Bp/4 <= 16), and whole warps stride together so the row-wide
 // ballot always has all 32 lanes.
@@ -524,7 +555,7 @@ __global__ void __launch_bounds__(kCopyThreads)
     batch_init_kernel(int32_t n, int B, int lq, int K, int c0, const int32_t *__restrict__ perm,
                       const int32_t *__restrict__ rowoff, const int32_t *__restrict__ odeg,
                       const float *__restrict__ rsum, const float *__restrict__ tele_old,
-                      float uniform, float one_minus_d, float *__restrict__ S,
+                      float uniform, float one_minus_d, bool all_rows, float *__restrict__ S,
                       float *__restrict__ C, float *__restrict__ base, uint8_t *__restrict__ tflag) {
   const int64_t total = static_cast<int64_t>(n) << lq;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -556,14 +587,16 @@ __global__ void __launch_bounds__(kCopyThreads)
     const bool row_nz = (__ballot_sync(0xffffffffu, nz) & grp_mask) != 0u;
     if (live) {
       const int64_t o = 4 * i;  // = u * Bp + 4 * q
-      *reinterpret_cast<float4 *>(S + o) = make_float4(t[0], t[1], t[2], t[3]);
-      *reinterpret_cast<float4 *>(C + o) =
-          make_float4(__fdiv_rn(t[0], denom), __fdiv_rn(t[1], denom), __fdiv_rn(t[2], denom),
-                      __fdiv_rn(t[3], denom));
-      if (row_nz)
+      if (row_nz || all_rows)
+        *reinterpret_cast<float4 *>(S + o) = make_float4(t[0], t[1], t[2], t[3]);
+      if (row_nz) {
+        *reinterpret_cast<float4 *>(C + o) =
+            make_float4(__fdiv_rn(t[0], denom), __fdiv_rn(t[1], denom), __fdiv_rn(t[2], denom),
+                        __fdiv_rn(t[3], denom));
         *reinterpret_cast<float4 *>(base + o) =
             make_float4(__fmul_rn(one_minus_d, t[0]), __fmul_rn(one_minus_d, t[1]),
                         __fmul_rn(one_minus_d, t[2]), __fmul_rn(one_minus_d, t[3]));
+      }
       if (q == 0) tflag[u] = row_nz ? 1 : 0;
     }
   }
@@ -720,9 +753,20 @@ int64_t HostBytes(int iters) {
   return kHostTraceOff + sizeof(double) * static_cast<int64_t>(std::max(iters, 1)) * kMaxTile;
 }
 
+// Long rows are cut so that the grid's warps (148 x 64) get about 16 tasks
+// each, in segments of 128 to 1024 entries: a warp gathers 128 / L rows at a
+// time, so a row of 4095 entries taken whole kept one warp busy for longer
+// than the rest of a small graph's sweep (300,007 vertices, 3.3 M edges, 16
+// columns: 131 us a sweep; 62 in segments).
+RowClasses BatchClasses(int64_t m) {
+  int32_t seg = 128;
+  while (seg < 1024 && seg < m / (148 * 64 * 16)) seg *= 2;
+  return RowClasses{seg, {128, 64, 32, 16, 8}};
+}
+
 // Buffers for tiles up to kMaxTile columns and a grid of up to nblocks.
-cudaError_t EnsureBatchBuffers(const DeviceGraph &g, BatchScratch &bs, int nblocks, int iters,
-                               std::string *err) {
+cudaError_t EnsureBatchBuffers(DeviceGraph &g, BatchScratch &bs, int nblocks, int iters,
+                               cudaStream_t s, std::string *err) {
   const int64_t n = g.n;
   const int64_t cells = n * kMaxTile;
   if (!bs.S || bs.cap_cells < cells) {
@@ -738,7 +782,7 @@ cudaError_t EnsureBatchBuffers(const DeviceGraph &g, BatchScratch &bs, int nbloc
     PB_TRY(GrowB(&bs.base, &c3, cells));
     bs.cap_cells = cells;
   }
-  const int ngroups = (nblocks + kReduceGroup - 1) / kReduceGroup;
+  const int ngroups = (nblocks + kColGroup - 1) / kColGroup;
   PB_TRY(GrowB(&bs.part1, &bs.cap_part, static_cast<int64_t>(nblocks) * kMaxTile));
   if (!bs.part2 || bs.cap_groups < ngroups + 1) {
     int64_t c = 0;
@@ -751,7 +795,10 @@ cudaError_t EnsureBatchBuffers(const DeviceGraph &g, BatchScratch &bs, int nbloc
   }
   PB_TRY(GrowB(&bs.trace, &bs.cap_trace, static_cast<int64_t>(std::max(iters, 1)) * kMaxTile));
   if (!bs.sweeps) PB_TRY(cudaMalloc(&bs.sweeps, sizeof(int32_t) * kMaxTile));
-  PB_TRY(GrowB(&bs.seg_partial, &bs.cap_seg, std::max<int64_t>(g.num_segments, 1) * kMaxTile));
+  if (!g.batch_tasks.ready)
+    PB_TRY(BuildRowTasks(static_cast<int32_t>(n), g.rowoff, true, BatchClasses(g.m), &g.batch_tasks, s));
+  PB_TRY(GrowB(&bs.seg_partial, &bs.cap_seg,
+               std::max<int64_t>(g.batch_tasks.task_start[1], 1) * kMaxTile));
   PB_TRY(GrowB(&bs.tflag, &bs.cap_flag, n));
   if (!bs.ctl) PB_TRY(cudaMalloc(&bs.ctl, sizeof(BatchCtl)));
   const int64_t host_need = HostBytes(iters);
@@ -774,7 +821,7 @@ int WidthIndex(int Bp) { return Bp == 8 ? 0 : Bp == 16 ? 1 : Bp == 32 ? 2 : 3; }
 // half the tile width, the loop stops, the survivors are repacked into the
 // narrowest tile that holds them, and sweeping resumes there (retired
 // columns' scores are written out at the end of the phase they retired in).
-cudaError_t SolveTile(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s, int max_iters,
+cudaError_t SolveTile(DeviceGraph &g, BatchScratch &bs, cudaStream_t s, int max_iters,
                       double epsilon, float damping, int K, int c0, int B, int Bp,
                       const BatchSchedule &sched, const float *tele_old, float *out_old,
                       int32_t *sweeps_tile, double *trace_tile, float *sweep_ms,
@@ -782,17 +829,18 @@ cudaError_t SolveTile(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s, in
   const int64_t n = g.n;
   const void *fn0 = BatchSweepKernel(g, Bp);
   const int nblocks0 = GridFor(fn0);
-  PB_TRY(EnsureBatchBuffers(g, bs, nblocks0, max_iters, err));
+  PB_TRY(EnsureBatchBuffers(g, bs, nblocks0, max_iters, s, err));
+  const RowTasks &rt = g.batch_tasks;
   const int lq = Log2(Bp / 4);
   const unsigned ib = CopyGrid(n << lq);
   const float uniform = 1.0f / static_cast<float>(n);
   const float omd = 1.0f - damping;
   if (g.weighted)
-    batch_init_kernel<true, false><<<ib, kCopyThreads, 0, s>>>(static_cast<int32_t>(n), B, lq, K, c0, g.perm, g.rowoff, g.odeg, g.rsum, tele_old, uniform, omd, bs.S, bs.C[0], bs.base, bs.tflag);
+    batch_init_kernel<true, false><<<ib, kCopyThreads, 0, s>>>(static_cast<int32_t>(n), B, lq, K, c0, g.perm, g.rowoff, g.odeg, g.rsum, tele_old, uniform, omd, max_iters == 0, bs.S, bs.C[0], bs.base, bs.tflag);
   else if (g.directed)
-    batch_init_kernel<false, true><<<ib, kCopyThreads, 0, s>>>(static_cast<int32_t>(n), B, lq, K, c0, g.perm, g.rowoff, g.odeg, g.rsum, tele_old, uniform, omd, bs.S, bs.C[0], bs.base, bs.tflag);
+    batch_init_kernel<false, true><<<ib, kCopyThreads, 0, s>>>(static_cast<int32_t>(n), B, lq, K, c0, g.perm, g.rowoff, g.odeg, g.rsum, tele_old, uniform, omd, max_iters == 0, bs.S, bs.C[0], bs.base, bs.tflag);
   else
-    batch_init_kernel<false, false><<<ib, kCopyThreads, 0, s>>>(static_cast<int32_t>(n), B, lq, K, c0, g.perm, g.rowoff, g.odeg, g.rsum, tele_old, uniform, omd, bs.S, bs.C[0], bs.base, bs.tflag);
+    batch_init_kernel<false, false><<<ib, kCopyThreads, 0, s>>>(static_cast<int32_t>(n), B, lq, K, c0, g.perm, g.rowoff, g.odeg, g.rsum, tele_old, uniform, omd, max_iters == 0, bs.S, bs.C[0], bs.base, bs.tflag);
   PB_TRY(cudaGetLastError());
   *launches += 1;
 
@@ -817,8 +865,8 @@ cudaError_t SolveTile(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s, in
   while (true) {
     const void *fn = BatchSweepKernel(g, tile_bp);
     const int nblocks = GridFor(fn);
-    PB_TRY(EnsureBatchBuffers(g, bs, nblocks, max_iters, err));
-    const int ngroups = (nblocks + kReduceGroup - 1) / kReduceGroup;
+    PB_TRY(EnsureBatchBuffers(g, bs, nblocks, max_iters, s, err));
+    const int ngroups = (nblocks + kColGroup - 1) / kColGroup;
     const unsigned long long active0 = (nact == 64) ? ~0ull : ((1ull << nact) - 1ull);
     batch_phase_begin_kernel<<<8, 256, 0, s>>>(bs.ctl, active0, loops, loops >= max_iters ? 1 : 0,
                                                bs.tick1, ngroups, bs.sweeps, bs.trace,
@@ -840,12 +888,12 @@ cudaError_t SolveTile(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s, in
     a.S = S;
     a.C0 = Cpair[0];
     a.C1 = Cpair[1];
-    a.nseg = static_cast<int32_t>(g.num_segments);
-    a.hub_rows = static_cast<int32_t>(g.num_hub_rows);
+    a.nseg = rt.task_start[1];
+    a.segment = rt.segment;
+    a.long_rows = rt.row_start[1];
     a.zero_start = static_cast<int32_t>(g.bin_row_start[kBinZero]);
-    a.seg_row = g.seg_row;
-    a.seg_first = g.seg_first;
-    a.hub_ticket = g.hub_ticket;
+    a.seg = rt.seg;
+    a.ticket = rt.ticket;
     a.seg_partial = bs.seg_partial;
     a.part1 = bs.part1;
     a.part2 = bs.part2;
@@ -966,7 +1014,7 @@ cudaError_t SolveTile(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s, in
 // column-sweep; then, at that width, tries half and twice the default
 // short-row length and L1 budgets of 64 and 160 KB, one knob after the
 // other, keeping a change only when it is faster.
-cudaError_t TuneTile(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s, float damping,
+cudaError_t TuneTile(DeviceGraph &g, BatchScratch &bs, cudaStream_t s, float damping,
                      int ncols, const float *tele_old, std::string *err) {
   std::vector<int32_t> sw(kMaxTile);
   auto time_one = [&](int w, const BatchSchedule &sch, double *per_col_sweep) {
@@ -1071,7 +1119,7 @@ void FreeBatchScratch(BatchScratch *b) {
   b->tuned_graph = nullptr;
 }
 
-cudaError_t SolveBatched(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s,
+cudaError_t SolveBatched(DeviceGraph &g, BatchScratch &bs, cudaStream_t s,
                          int max_iters, double epsilon, float damping, int ncols,
                          const float *tele_old, float *out_old, int32_t *sweeps_out,
                          double *err_trace, double *ms_sweep, double *ms_total,

@@ -81,7 +81,7 @@ BatchSchedule ResolveSchedule(const BatchScratch &bs, int Bp);
 // ids, device; nullptr = every column uniform 1/N) into out (N x ncols,
 // original ids, device), one column tile at a time.  sweeps_out / err_trace
 // are host arrays (nullable) laid out as in pr_gpu_run.
-cudaError_t SolveBatched(const DeviceGraph &g, BatchScratch &bs, cudaStream_t s,
+cudaError_t SolveBatched(DeviceGraph &g, BatchScratch &bs, cudaStream_t s,
                          int max_iters, double epsilon, float damping, int ncols,
                          const float *tele_old, float *out_old, int32_t *sweeps_out,
                          double *err_trace, double *ms_sweep, double *ms_total,

@@ -97,6 +97,7 @@ struct DeviceGraph {
   // tasks of the resident solves over the in-rows and (directed: adjoint)
   // the out-rows, built by the first such solve
   RowTasks in_tasks, out_tasks;
+  RowTasks batch_tasks;      // long in-rows of batched solves, by their first one
   int64_t tile_entries = 0;  // in-entries of the first kResidentTile vertices
 };
 

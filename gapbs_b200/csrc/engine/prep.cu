@@ -228,6 +228,7 @@ void FreeDeviceGraph(DeviceGraph *g) {
     if (p) cudaFree(p);
   FreeRowTasks(&g->in_tasks);
   FreeRowTasks(&g->out_tasks);
+  FreeRowTasks(&g->batch_tasks);
   BinConfig keep = g->bins;
   *g = DeviceGraph();
   g->bins = keep;
