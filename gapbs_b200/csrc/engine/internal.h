@@ -80,6 +80,7 @@ struct DeviceGraph {
   int32_t *orowoff = nullptr;  // directed: renumbered out-CSR (adjoint)
   int32_t *ocol = nullptr;
   float *wout = nullptr;       // weighted: w(v->u) aligned with the out rows
+  unsigned *weight_flag = nullptr;  // weighted: validation flag of new weights
   int32_t *orig_out_off = nullptr;  // the caller's out-offsets (original ids):
                                     // entry j of renumbered out-row v sits at
                                     // orig_out_off[perm[v]] + j in the caller's CSR

@@ -700,6 +700,9 @@ int SolveAdjoint(pr_gpu_t *h, int max_iters, double epsilon, float damping, cons
     return PR_GPU_OK;
   }
   // undirected graphs only (UseResident)
+  if (grad_ew && !g.in_tasks.ready)  // the gradient kernel's split of the rows
+    PR_CHECK(h, prgpu::BuildRowTasks(static_cast<int32_t>(g.n), g.rowoff, true,
+                                     prgpu::ClassesFor(g.m, g.weighted), &g.in_tasks, h->stream));
   int32_t task_start[prgpu::kNumBins + 1];
   prgpu::PullTasks(g, task_start);
   prgpu::PullArgs probe;

@@ -23,7 +23,9 @@
 #include <string>
 #include <vector>
 
+#include "common.cuh"
 #include "internal.h"
+#include "resident.h"
 
 namespace prgpu {
 
@@ -58,9 +60,16 @@ __global__ void validate_ids_kernel(int64_t m, int64_t n, const int32_t *nbr,
 
 __global__ void validate_weights_kernel(int64_t m, const float *w, unsigned *flag) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const float x = w[i];
-  if (!(x > 0.f) || !isfinite(x)) atomicOr(flag, kBadWeight);
+  if (4 * i >= m) return;
+  // the caller's weights may start at any float
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (4 * i + k < m) {
+      const float x = w[4 * i + k];
+      bad |= !(x > 0.f) || !isfinite(x);
+    }
+  if (bad) atomicOr(flag, kBadWeight);
 }
 
 // Out-rows must be strictly increasing for the weight lookup.
@@ -97,8 +106,7 @@ __global__ void renumber_rows_kernel(int64_t n, const int32_t *__restrict__ perm
                                      const int32_t *__restrict__ src_nbr,
                                      const int32_t *__restrict__ dst_off,
                                      const int32_t *__restrict__ translate,
-                                     int32_t *dst_nbr, const float *__restrict__ src_w,
-                                     float *dst_w, int32_t *dst_pos) {
+                                     int32_t *dst_nbr) {
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n) return;
@@ -106,12 +114,8 @@ __global__ void renumber_rows_kernel(int64_t n, const int32_t *__restrict__ perm
   const int32_t s = src_off[v], len = src_off[v + 1] - s;
   const int32_t d = dst_off[warp];
   for (int32_t j = lane; j < len; j += 32) {
-    if (dst_nbr) {
-      const int32_t x = src_nbr[s + j];
-      dst_nbr[d + j] = translate ? translate[x] : x;
-    }
-    if (dst_w) dst_w[d + j] = src_w[s + j];
-    if (dst_pos) dst_pos[d + j] = s + j;
+    const int32_t x = src_nbr[s + j];
+    dst_nbr[d + j] = translate ? translate[x] : x;
   }
 }
 
@@ -123,15 +127,46 @@ __global__ void out_degree_kernel(int64_t n, const int32_t *perm, const int32_t 
   odeg[u] = out_off[v + 1] - out_off[v];
 }
 
-// S_v per renumbered vertex, summed in double in row order then rounded.
-__global__ void row_weight_sum_kernel(int64_t n, const int32_t *perm, const int32_t *out_off,
-                                      const float *ew, float *rsum) {
-  const int64_t u = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (u >= n) return;
-  const int32_t v = perm[u];
+// The out-row at position p of the tasks' order, v, by T threads: its weights
+// from the caller's CSR to wout, and S_v, their sum in double (a fixed tree)
+// rounded once.  Rows of at least 1,024 entries get a block each, as the
+// longest would keep a single thread (1.5 ms at Kronecker 2^20) or warp busy
+// long after the others are done.
+struct RowWeightArgs {
+  const int32_t *__restrict__ order;
+  const int32_t *__restrict__ perm;
+  const int32_t *__restrict__ orig_off;
+  const int32_t *__restrict__ orow;
+  const float *__restrict__ w;
+  float *wout;
+  float *rsum;
+};
+
+template <int T>
+__device__ __forceinline__ void row_weights(const RowWeightArgs &a, int p, int t, double *sred) {
+  const int32_t v = a.order ? a.order[p] : p;
+  const int32_t s = a.orig_off[a.perm[v]], d = a.orow[v];
+  const int32_t len = a.orow[v + 1] - d;
   double acc = 0;
-  for (int32_t e = out_off[v]; e < out_off[v + 1]; e++) acc += ew[e];
-  rsum[u] = static_cast<float>(acc);
+#pragma unroll 4
+  for (int32_t j = t; j < len; j += T) {
+    const float x = a.w[s + j];
+    a.wout[d + j] = x;
+    acc += x;
+  }
+  acc = T == 32 ? warp_sum_d(acc) : block_sum_d<T>(acc, sred);
+  if (t == 0) a.rsum[v] = static_cast<float>(acc);
+}
+
+__global__ void __launch_bounds__(1024) row_weights_long_kernel(const RowWeightArgs a) {
+  __shared__ double sred[32];
+  row_weights<1024>(a, blockIdx.x, threadIdx.x, sred);
+}
+
+__global__ void __launch_bounds__(256)
+row_weights_kernel(const RowWeightArgs a, int32_t first, int32_t n) {
+  const int64_t p = first + ((static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5);
+  if (p < n) row_weights<32>(a, static_cast<int>(p), threadIdx.x & 31, nullptr);
 }
 
 // In-edge weights aligned with the renumbered in-CSR: entry j of new row u is
@@ -191,13 +226,38 @@ inline unsigned Blocks(int64_t count, int threads) {
   return static_cast<unsigned>((count + threads - 1) / threads);
 }
 
-// win[j] = w[win_pos[j]] over the renumbered in-CSR entries.
-__global__ void gather_weights_kernel(int64_t m, const int32_t *__restrict__ pos,
-                                      const float *__restrict__ w, float *out) {
+// win[j] = w[win_pos[j]] over the renumbered in-CSR entries, four a thread so
+// that their random reads are in flight together (both arrays are padded to
+// whole float4; a padding entry has position -1 or is never read).
+__global__ void gather_weights_kernel(int64_t m, const int4 *__restrict__ pos,
+                                      const float *__restrict__ w, float4 *out) {
   const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (j >= m) return;
-  const int32_t p = pos[j];
-  out[j] = p >= 0 ? w[p] : 0.f;
+  if (4 * j >= m) return;
+  int4 p = pos[j];
+  if (4 * j + 1 >= m) p.y = -1;
+  if (4 * j + 2 >= m) p.z = -1;
+  if (4 * j + 3 >= m) p.w = -1;
+  const float x = p.x >= 0 ? w[p.x] : 0.f, y = p.y >= 0 ? w[p.y] : 0.f;
+  const float z = p.z >= 0 ? w[p.z] : 0.f, q = p.w >= 0 ? w[p.w] : 0.f;
+  out[j] = make_float4(x, y, z, q);
+}
+
+// rsum and wout from the weights in the caller's out-CSR order.
+cudaError_t ApplyRowWeights(DeviceGraph *g, const float *d_w, cudaStream_t s) {
+  const int32_t n = static_cast<int32_t>(g->n);
+  const int32_t *oro = g->directed ? g->orowoff : g->rowoff;
+  RowTasks &rt = g->directed ? g->out_tasks : g->in_tasks;
+  if (!rt.ready) {
+    cudaError_t e = BuildRowTasks(n, oro, !g->directed, ClassesFor(g->m, true), &rt, s);
+    if (e != cudaSuccess) return e;
+  }
+  const RowWeightArgs a{rt.order, g->perm, g->orig_out_off, oro, d_w, g->wout, g->rsum};
+  const int32_t nlong = rt.row_start[1];
+  if (nlong) row_weights_long_kernel<<<nlong, 1024, 0, s>>>(a);
+  if (n > nlong)
+    row_weights_kernel<<<static_cast<unsigned>((static_cast<int64_t>(n - nlong) + 7) / 8), 256, 0, s>>>(
+        a, nlong, n);
+  return cudaGetLastError();
 }
 
 std::string FlagText(unsigned f) {
@@ -223,7 +283,7 @@ cudaError_t Alloc(T **p, int64_t count) {
 void FreeDeviceGraph(DeviceGraph *g) {
   void *ptrs[] = {g->rowoff, g->col, g->win, g->win_pos, g->odeg, g->rsum, g->orowoff, g->ocol,
                   g->wout, g->orig_out_off, g->perm, g->inv, g->seg_row, g->seg_first, g->hub_ticket,
-                  g->seg_partial};
+                  g->seg_partial, g->weight_flag};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   FreeRowTasks(&g->in_tasks);
@@ -280,7 +340,7 @@ cudaError_t BuildDeviceGraph(DeviceGraph *g, int64_t n, int64_t m,
     if (m) validate_ids_kernel<<<Blocks(m, T), T, 0, s>>>(m, n, d_out_nbr, d_flag);
   }
   if (g->weighted) {
-    if (m) validate_weights_kernel<<<Blocks(m, T), T, 0, s>>>(m, d_ew, d_flag);
+    if (m) validate_weights_kernel<<<Blocks((m + 3) / 4, T), T, 0, s>>>(m, d_ew, d_flag);
     validate_sorted_kernel<<<Blocks(n, T), T, 0, s>>>(n, d_out_off, d_out_nbr, d_flag);
   }
   PR_TRY(cudaGetLastError());
@@ -326,7 +386,7 @@ cudaError_t BuildDeviceGraph(DeviceGraph *g, int64_t n, int64_t m,
   PR_TRY(Alloc(&g->col, m_pad));
   PR_TRY(cudaMemsetAsync(g->col, 0, sizeof(int32_t) * m_pad, s));
   renumber_rows_kernel<<<Blocks(n * 32, T), T, 0, s>>>(n, g->perm, d_in_off, d_in_nbr, g->rowoff,
-                                                       g->inv, g->col, nullptr, nullptr, nullptr);
+                                                       g->inv, g->col);
   PR_TRY(cudaGetLastError());
 
   if (directed) {
@@ -339,34 +399,29 @@ cudaError_t BuildDeviceGraph(DeviceGraph *g, int64_t n, int64_t m,
     PR_TRY(Alloc(&g->ocol, m_pad));
     PR_TRY(cudaMemsetAsync(g->ocol, 0, sizeof(int32_t) * m_pad, s));
     renumber_rows_kernel<<<Blocks(n * 32, T), T, 0, s>>>(n, g->perm, d_out_off, d_out_nbr,
-                                                         g->orowoff, g->inv, g->ocol, nullptr,
-                                                         nullptr, nullptr);
+                                                         g->orowoff, g->inv, g->ocol);
     PR_TRY(cudaGetLastError());
   }
+
+  PR_TRY(Alloc(&g->orig_out_off, n + 1));
+  PR_TRY(cudaMemcpyAsync(g->orig_out_off, d_out_off, sizeof(int32_t) * (n + 1),
+                         cudaMemcpyDeviceToDevice, s));
 
   // 4. weights
   if (g->weighted) {
     PR_TRY(Alloc(&g->rsum, n));
-    row_weight_sum_kernel<<<Blocks(n, T), T, 0, s>>>(n, g->perm, d_out_off, d_ew, g->rsum);
     PR_TRY(Alloc(&g->win, m_pad));
     PR_TRY(cudaMemsetAsync(g->win, 0, sizeof(float) * m_pad, s));
     PR_TRY(Alloc(&g->win_pos, m_pad));
     in_weight_kernel<<<Blocks(n * 32, T), T, 0, s>>>(n, g->perm, d_in_off, d_in_nbr, d_out_off,
                                                      d_out_nbr, d_ew, g->rowoff, g->win,
                                                      g->win_pos, d_flag);
-    const int32_t *oro = directed ? g->orowoff : g->rowoff;
     PR_TRY(Alloc(&g->wout, m_pad));
     PR_TRY(cudaMemsetAsync(g->wout, 0, sizeof(float) * m_pad, s));
-    renumber_rows_kernel<<<Blocks(n * 32, T), T, 0, s>>>(n, g->perm, d_out_off, d_out_nbr, oro,
-                                                         g->inv, nullptr, d_ew, g->wout,
-                                                         nullptr);
-    PR_TRY(cudaGetLastError());
+    PR_TRY(ApplyRowWeights(g, d_ew, s));
+    PR_TRY(Alloc(&g->weight_flag, 1));
     PR_TRY(cudaMemcpyAsync(&flag, d_flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   }
-
-  PR_TRY(Alloc(&g->orig_out_off, n + 1));
-  PR_TRY(cudaMemcpyAsync(g->orig_out_off, d_out_off, sizeof(int32_t) * (n + 1),
-                         cudaMemcpyDeviceToDevice, s));
 
   // 5. bins and hub segments
   PR_TRY(Alloc(&d_bins, kNumBins + 1));
@@ -421,34 +476,26 @@ cudaError_t UpdateDeviceWeights(DeviceGraph *g, const float *d_w, cudaStream_t s
     *err = "the graph on the device has no edge weights";
     return cudaErrorInvalidValue;
   }
-  const int64_t n = g->n, m = g->m;
+  const int64_t m = g->m;
   const int T = 256;
-  unsigned *d_flag = nullptr;
-  auto cleanup = [&]() {
-    if (d_flag) cudaFree(d_flag);
-    d_flag = nullptr;
-  };
-  PR_TRY(Alloc(&d_flag, 1));
-  PR_TRY(cudaMemsetAsync(d_flag, 0, sizeof(unsigned), s));
-  if (m) validate_weights_kernel<<<Blocks(m, T), T, 0, s>>>(m, d_w, d_flag);
+  auto cleanup = [] {};
+  PR_TRY(cudaMemsetAsync(g->weight_flag, 0, sizeof(unsigned), s));
+  if (m) validate_weights_kernel<<<Blocks((m + 3) / 4, T), T, 0, s>>>(m, d_w, g->weight_flag);
   PR_TRY(cudaGetLastError());
   unsigned flag = 0;
-  PR_TRY(cudaMemcpyAsync(&flag, d_flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+  PR_TRY(cudaMemcpyAsync(&flag, g->weight_flag, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
   PR_TRY(cudaStreamSynchronize(s));
   if (flag) {
     *err = "invalid edge weights:" + FlagText(flag);
-    cleanup();
     return cudaErrorInvalidValue;
   }
   // the same three arrays BuildDeviceGraph derives from the weights
-  row_weight_sum_kernel<<<Blocks(n, T), T, 0, s>>>(n, g->perm, g->orig_out_off, d_w, g->rsum);
-  if (m) gather_weights_kernel<<<Blocks(m, T), T, 0, s>>>(m, g->win_pos, d_w, g->win);
-  const int32_t *oro = g->directed ? g->orowoff : g->rowoff;
-  renumber_rows_kernel<<<Blocks(n * 32, T), T, 0, s>>>(n, g->perm, g->orig_out_off, nullptr, oro,
-                                                       nullptr, nullptr, d_w, g->wout, nullptr);
+  PR_TRY(ApplyRowWeights(g, d_w, s));
+  if (m)
+    gather_weights_kernel<<<Blocks((m + 3) / 4, T), T, 0, s>>>(
+        m, reinterpret_cast<const int4 *>(g->win_pos), d_w, reinterpret_cast<float4 *>(g->win));
   PR_TRY(cudaGetLastError());
   PR_TRY(cudaStreamSynchronize(s));
-  cleanup();
   return cudaSuccess;
 }
 
