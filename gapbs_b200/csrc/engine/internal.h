@@ -218,16 +218,16 @@ struct CcScratch {
 void FreeCcScratch(CcScratch *c);
 
 // Breadth-first search (bfs.cu).  Work arrays kept between calls.
+struct BfsResult {  // page-locked, written by the device
+  int32_t nlog, error;
+};
 struct BfsScratch {
   int32_t *parent = nullptr, *queue[2] = {nullptr, nullptr};
   unsigned *bm[2] = {nullptr, nullptr};
-  int64_t *deg = nullptr, *eoff = nullptr, *sums = nullptr;
-  void *ctl = nullptr;  // the search's control block (bfs.cu)
+  int32_t *eoff = nullptr, *sums = nullptr;
+  void *ctl = nullptr;  // barrier, counters and step log (bfs.cu)
+  BfsResult *res = nullptr;
   int64_t cap_n = 0;
-  // the search loop graph and the launch plan it was captured with
-  cudaGraphExec_t exec = nullptr;
-  cudaStream_t cap_stream = nullptr;
-  std::vector<unsigned char> plan;
 };
 struct BfsStep {
   const char *kind;  // "i", "td", "e", "bu", "c" as the reference logs them

@@ -64,7 +64,7 @@ struct pr_gpu {
   // resident solves: barrier state, and the page-locked block they report in
   // (ResidentResult, then kHostTrace doubles of trace)
   static constexpr int kHostTrace = 4096;
-  prgpu::ResidentCtl *rctl = nullptr;
+  prgpu::GridBarrier *rctl = nullptr;
   prgpu::ResidentResult *rres = nullptr;
   prgpu::CcScratch cc;    // connected-components work arrays
   prgpu::BfsScratch bfs;  // breadth-first-search work arrays
@@ -391,14 +391,14 @@ int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float da
   prgpu::ResidentArgs a;
   std::memset(&a, 0, sizeof(a));
   a.tile = static_cast<int32_t>(std::min<int64_t>(g.n, prgpu::kResidentTile) & ~int64_t(3));
-  int grid = static_cast<int>(
+  const int grid = static_cast<int>(
       std::max<int64_t>(1, std::min<int64_t>(sms, g.m / prgpu::kResidentEntriesPerCta)));
   int rc = EnsureScratch(h, g.n, 1, 2 * grid, max_iters);
   if (rc) return rc;
   Scratch &sc = h->sc;
   if (!h->rctl) {
-    PR_CHECK(h, cudaMalloc(&h->rctl, sizeof(prgpu::ResidentCtl)));
-    PR_CHECK(h, cudaMemsetAsync(h->rctl, 0, sizeof(prgpu::ResidentCtl), s));
+    PR_CHECK(h, cudaMalloc(&h->rctl, sizeof(prgpu::GridBarrier)));
+    PR_CHECK(h, cudaMemsetAsync(h->rctl, 0, sizeof(prgpu::GridBarrier), s));
   }
   if (!h->rres)
     PR_CHECK(h, cudaHostAlloc(reinterpret_cast<void **>(&h->rres),
@@ -446,19 +446,11 @@ int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float da
   PR_CHECK(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    static_cast<int>(smem)));
   PR_CHECK(h, cudaEventRecord(h->ev[0], s));
-  void *params[] = {&a};
-  cudaError_t le = cudaSuccess;
-  for (;; grid /= 2) {
-    le = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(prgpu::kResidentThreads), params, smem, s);
-    // a stream that may use part of the GPU only: any grid size solves
-    if (le != cudaErrorCooperativeLaunchTooLarge || grid == 1) break;
-    cudaGetLastError();
-  }
-  PR_CHECK(h, le);
+  PR_CHECK(h, prgpu::LaunchGrid(fn, grid, prgpu::kResidentThreads, &a, smem, s));
   PR_CHECK(h, cudaEventRecord(h->ev[3], s));
   PR_CHECK(h, cudaStreamSynchronize(s));
   if (h->rres->failed) {
-    PR_CHECK(h, cudaMemsetAsync(h->rctl, 0, sizeof(prgpu::ResidentCtl), s));
+    PR_CHECK(h, cudaMemsetAsync(h->rctl, 0, sizeof(prgpu::GridBarrier), s));
     return SetErr(h, PR_GPU_ECUDA, "a grid barrier of the solve ran out of its wait");
   }
   const int sweeps = h->rres->sweeps;

@@ -41,6 +41,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "grid_barrier.cuh"
 #include "resident.h"
 
 namespace prgpu {
@@ -51,9 +52,6 @@ constexpr int kThreads = kResidentThreads;
 constexpr int kWarps = kThreads / 32;
 static_assert(kWarps == 32, "one warp sums the warps' partials");
 constexpr unsigned kFull = 0xffffffffu;
-// polls of the barrier before a CTA gives up (about 10 s)
-constexpr unsigned kMaxPolls = 1u << 24;
-
 // Entry v of cin: from shared memory below `tile`, else from L2 (other CTAs
 // wrote it in the sweep before, and L1 is not coherent within a launch).
 // v == -1 reads the zero slot in front of the tile.  Both loads are predicated,
@@ -78,37 +76,10 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
-}
-
-// Thread 0 of every CTA arrives and waits until all have arrived `round`
-// times; false when the wait ran out.  Called by all threads; everything
-// written before it by any CTA is visible after it (to loads that do not
-// hit L1).
-__device__ __forceinline__ bool grid_barrier(ResidentCtl *ctl, unsigned round, int *s_ok) {
-  __syncthreads();
-  if (gridDim.x == 1) return true;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(&ctl->arrived, 1u);
-    const unsigned want = round * gridDim.x;
-    unsigned polls = 0;
-    while (ld_acquire(&ctl->arrived) < want && ++polls < kMaxPolls) {
-    }
-    *s_ok = polls < kMaxPolls;
-    __threadfence();
-  }
-  __syncthreads();
-  return *s_ok != 0;
 }
 
 // Sum of the CTAs' partials in a fixed order, by one warp; valid in lane 0.
@@ -423,15 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_solve_kernel(const Resid
       a.out_old[v] = KIND == kKindAdjoint ? __fmul_rn(a.one_minus_d, x) : x;
     }
   }
-  // the last CTA to leave makes the barrier ready for the next solve: all
-  // have passed their last wait by then
-  if (threadIdx.x == 0) {
-    const unsigned left = atomicAdd(&a.ctl->left, 1u);
-    if (left == gridDim.x - 1) {
-      a.ctl->arrived = 0;
-      a.ctl->left = 0;
-    }
-  }
+  leave_grid(a.ctl);
 }
 
 template <bool W, bool DIR>
@@ -512,6 +475,17 @@ cudaError_t SortRows(int32_t n, const int32_t *rowoff, int32_t *order, cudaStrea
 }
 
 }  // namespace
+
+cudaError_t LaunchGrid(const void *fn, int grid, int threads, void *args, size_t smem,
+                       cudaStream_t s) {
+  void *params[] = {args};
+  for (;; grid /= 2) {
+    const cudaError_t e =
+        cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), params, smem, s);
+    if (e != cudaErrorCooperativeLaunchTooLarge || grid == 1) return e;
+    cudaGetLastError();
+  }
+}
 
 void FreeRowTasks(RowTasks *r) {
   for (void *p : {static_cast<void *>(r->order), static_cast<void *>(r->seg),

@@ -16,11 +16,17 @@ constexpr int kResidentThreads = 1024;
 // solve: 88 with 20 CTAs, 96 with 5, 137 with one).
 constexpr int64_t kResidentEntriesPerCta = 1024;
 
-// Barrier state, zero between solves.
-struct ResidentCtl {
-  unsigned arrived;  // CTAs that arrived, all rounds of a solve together
-  unsigned left;     // CTAs that left the solve
+// State of a barrier between a launch's CTAs (grid_barrier.cuh), zero between
+// launches; a launch whose wait ran out leaves it to be cleared.
+struct GridBarrier {
+  unsigned arrived;  // CTAs that arrived, all rounds of a launch together
+  unsigned left;     // CTAs that left the launch
 };
+
+// Cooperative launch of fn(args) on `grid` CTAs, or on fewer where the stream
+// may use part of the GPU only (the kernels take any grid size).
+cudaError_t LaunchGrid(const void *fn, int grid, int threads, void *args, size_t smem,
+                       cudaStream_t s);
 
 // What a solve tells the host (page-locked host memory).
 struct ResidentResult {
@@ -54,7 +60,7 @@ struct ResidentArgs {
   double epsilon;
   double *part;   // 2 x CTAs
   double *trace;  // max_iters
-  ResidentCtl *ctl;
+  GridBarrier *ctl;
   ResidentResult *res;
 };
 
