@@ -200,6 +200,16 @@ cudaError_t UpdateDeviceWeights(DeviceGraph *g, const float *d_w, cudaStream_t s
 // not used.
 cudaError_t VerifyResiduals(const DeviceGraph &g, const float *score_orig, float damping,
                             float *contrib, float *resid_orig, cudaStream_t s);
+// *out (host) = the double that adding resid[0 .. n) (floats >= 0, infinities
+// and NaN allowed) to 0.0 one after the other gives, bit for bit; returns
+// when it is there.
+struct VerifyScratch {
+  void *mem = nullptr;
+  size_t bytes = 0;
+};
+void FreeVerifyScratch(VerifyScratch *v);
+cudaError_t SumInOrder(int64_t n, const float *resid, VerifyScratch &v, double *out,
+                       cudaStream_t s);
 
 // The reference's -g / -u graph built on the device (generate.cu): CSR of
 // the symmetrised, squished graph in original ids, int32 offsets (n+1) and
