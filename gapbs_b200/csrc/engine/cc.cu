@@ -32,12 +32,14 @@
 #include <cstdint>
 #include <string>
 
+#include "grid_barrier.cuh"
 #include "internal.h"
 
 namespace prgpu {
 
 namespace {
 
+constexpr int kThreads = 1024, kCtasPerSm = 2;
 constexpr int kChaseLimit = 1 << 20;  // far above any tree depth reached
 
 __device__ __forceinline__ int ld_comp(const int *comp, int x) {
@@ -73,7 +75,7 @@ __device__ void cc_link(int u, int v, int *comp, int *err) {
   bool u_root = p1 == u;
   for (int it = 0; p1 != p2; it++) {
     if (it >= kChaseLimit) {
-      atomicExch(err, 1);
+      *err = 1;
       return;
     }
     const int high = max(p1, p2), low = min(p1, p2);
@@ -93,181 +95,189 @@ __device__ void cc_link(int u, int v, int *comp, int *err) {
   }
 }
 
-__global__ void cc_init_kernel(int32_t n, int *comp) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += stride)
-    comp[v] = static_cast<int>(v);
-}
+struct CcArgs {
+  int32_t n, active, long_rows;
+  const int32_t *__restrict__ ooff;
+  const int32_t *__restrict__ onbr;
+  const int32_t *__restrict__ ioff;  // directed graphs, else null
+  const int32_t *__restrict__ inbr;
+  const int32_t *__restrict__ perm;
+  const int32_t *__restrict__ inv;
+  int *comp, *root_min, *second;
+  int32_t *out_old;
+  GridBarrier *barrier;
+  int *err;  // page-locked: 1 an iteration limit, 2 a barrier wait ran out
+};
 
-// One sampling round (src/cc.cc:100-106): vertex u links with its r-th
+// First sampling round (src/cc.cc:100-106): vertex u links with its first
 // out-neighbour.  Each thread takes two vertices per pass and loads both
 // neighbour ids (random reads of the neighbour array, one HBM sector each)
-// before either link, so two such reads are in flight per thread.
-__global__ void cc_sample_kernel(int32_t n, const int32_t *__restrict__ off,
-                                 const int32_t *__restrict__ nbr, int r, int *comp, int *err) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t u = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < n;
-       u += 2 * stride) {
+// before either link, so two such reads are in flight per thread.  The second
+// neighbour, mostly in the same sector, is kept for the second round, which
+// then reads it in order (62 us a round at Kronecker 2^23 as random reads).
+__device__ __forceinline__ void sample_first(const CcArgs &a, int64_t gtid, int64_t stride) {
+  for (int64_t u = gtid; u < a.active; u += 2 * stride) {
     const int64_t u2 = u + stride;
-    const int s1 = off[u], e1 = off[u + 1];
+    const int s1 = a.ooff[u], e1 = a.ooff[u + 1];
     int s2 = 0, e2 = 0;
-    if (u2 < n) {
-      s2 = off[u2];
-      e2 = off[u2 + 1];
+    if (u2 < a.active) {
+      s2 = a.ooff[u2];
+      e2 = a.ooff[u2 + 1];
     }
-    const int v1 = s1 + r < e1 ? nbr[s1 + r] : -1;
-    const int v2 = s2 + r < e2 ? nbr[s2 + r] : -1;
-    if (v1 >= 0) cc_link(static_cast<int>(u), v1, comp, err);
-    if (v2 >= 0) cc_link(static_cast<int>(u2), v2, comp, err);
+    const int v1 = s1 < e1 ? a.onbr[s1] : -1;
+    const int v2 = s2 < e2 ? a.onbr[s2] : -1;
+    const int w1 = s1 + 1 < e1 ? a.onbr[s1 + 1] : -1;
+    const int w2 = s2 + 1 < e2 ? a.onbr[s2 + 1] : -1;
+    a.second[u] = w1;
+    if (u2 < a.active) a.second[u2] = w2;
+    if (v1 >= 0) cc_link(static_cast<int>(u), v1, a.comp, a.err);
+    if (v2 >= 0) cc_link(static_cast<int>(u2), v2, a.comp, a.err);
+  }
+}
+
+__device__ __forceinline__ void sample_second(const CcArgs &a, int64_t gtid, int64_t stride) {
+  for (int64_t u = gtid; u < a.active; u += stride) {
+    const int v = a.second[u];
+    if (v >= 0) cc_link(static_cast<int>(u), v, a.comp, a.err);
   }
 }
 
 // src/cc.cc:58-66.  No link runs during a compress, so roots are fixed and
 // every non-root x has comp[x] != x at all times: c == comp[c] holds exactly
 // when c is a root, whether comp[c] was read fresh or from L1.
-__global__ void cc_compress_kernel(int32_t n, int *comp, int *err) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += stride) {
-    int it = 0;
-    int c = ld_comp(comp, static_cast<int>(v));
-    int cc = ld_comp_cached(comp, c);
-    while (c != cc) {
-      if (++it >= kChaseLimit) {
-        atomicExch(err, 1);
-        break;
-      }
-      comp[v] = cc;
-      c = cc;
-      cc = ld_comp_cached(comp, c);
+__device__ __forceinline__ int compress_one(int v, int *comp, int *err) {
+  int it = 0;
+  int c = ld_comp(comp, v);
+  int cc = ld_comp_cached(comp, c);
+  while (c != cc) {
+    if (++it >= kChaseLimit) {
+      *err = 1;
+      break;
     }
+    comp[v] = cc;
+    c = cc;
+    cc = ld_comp_cached(comp, c);
   }
+  return c;
 }
 
-// Final phase: out-neighbours from index `skip` on and, for a directed graph,
-// all in-neighbours; vertices of component `giant` are skipped
-// (src/cc.cc:122-146).  Rows [row0, row1), one warp per vertex (the long
-// rows at the front of the degree-sorted mirror).
-__global__ void cc_finish_warp_kernel(int32_t row0, int32_t row1, const int32_t *__restrict__ ooff,
-                                      const int32_t *__restrict__ onbr,
-                                      const int32_t *__restrict__ ioff,
-                                      const int32_t *__restrict__ inbr, int skip, int giant,
-                                      int *comp, int *err) {
+// Final phase: out-neighbours from the third on and, for a directed graph,
+// all in-neighbours; vertices of the component of row 0 are skipped
+// (src/cc.cc:122-146).  A warp reads the components of 32 consecutive rows at
+// once, since nearly all are skipped, then takes the long rows left (the
+// front of the degree-sorted mirror) together and the others a lane each.
+__device__ __forceinline__ void link_rest(const CcArgs &a, int giant) {
   const int lane = threadIdx.x & 31;
-  const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t u = row0 + ((static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
-       u < row1; u += warps) {
-    if (ld_comp(comp, static_cast<int>(u)) == giant) continue;
-    for (int j = ooff[u] + skip + lane; j < ooff[u + 1]; j += 32)
-      cc_link(static_cast<int>(u), onbr[j], comp, err);
-    if (ioff)
-      for (int j = ioff[u] + lane; j < ioff[u + 1]; j += 32)
-        cc_link(static_cast<int>(u), inbr[j], comp, err);
-  }
-}
-
-// The same for rows [row0, row1), one thread per vertex (the short rows).
-__global__ void cc_finish_thread_kernel(int32_t row0, int32_t row1,
-                                        const int32_t *__restrict__ ooff,
-                                        const int32_t *__restrict__ onbr,
-                                        const int32_t *__restrict__ ioff,
-                                        const int32_t *__restrict__ inbr, int skip, int giant,
-                                        int *comp, int *err) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t u = row0 + static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < row1;
-       u += stride) {
-    if (ld_comp(comp, static_cast<int>(u)) == giant) continue;
-    for (int j = ooff[u] + skip; j < ooff[u + 1]; j++) cc_link(static_cast<int>(u), onbr[j], comp, err);
-    if (ioff)
-      for (int j = ioff[u]; j < ioff[u + 1]; j++) cc_link(static_cast<int>(u), inbr[j], comp, err);
-  }
-}
-
-// The last compress, fused with the ids mapped back: every vertex chases
-// to its root (as cc_compress_kernel) and offers its original id to the
-// root's minimum.  Members of the component of row 0 (the largest one; half
-// the graph on Kronecker inputs) are reduced per thread and per block first,
-// so its root takes one atomic per block instead of one per vertex.
-__global__ void __launch_bounds__(256) cc_compress_min_kernel(int32_t n, int *comp,
-                                                              const int32_t *__restrict__ perm,
-                                                              int *root_min, int *err) {
-  __shared__ int s_min[8];
-  const int giant = 0;  // row 0 is the root of its component
-  int local = INT_MAX;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t v = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; v < n; v += stride) {
-    int it = 0;
-    int c = ld_comp(comp, static_cast<int>(v));
-    int cc = ld_comp_cached(comp, c);
-    while (c != cc) {
-      if (++it >= kChaseLimit) {
-        atomicExch(err, 1);
-        break;
-      }
-      comp[v] = cc;
-      c = cc;
-      cc = ld_comp_cached(comp, c);
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+  for (int64_t b = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+       b << 5 < a.active; b += warps) {
+    const int u = static_cast<int>(b << 5) + lane;
+    const bool left = u < a.active && ld_comp(a.comp, u) != giant;
+    unsigned together = __ballot_sync(0xffffffffu, left && u < a.long_rows);
+    while (together) {
+      const int w = static_cast<int>(b << 5) + __ffs(together) - 1;
+      together &= together - 1;
+      for (int j = a.ooff[w] + 2 + lane; j < a.ooff[w + 1]; j += 32)
+        cc_link(w, a.onbr[j], a.comp, a.err);
+      if (a.ioff)
+        for (int j = a.ioff[w] + lane; j < a.ioff[w + 1]; j += 32)
+          cc_link(w, a.inbr[j], a.comp, a.err);
+      __syncwarp();
     }
-    if (c == giant) local = min(local, perm[v]);
-    else atomicMin(root_min + c, perm[v]);
+    if (left && u >= a.long_rows) {
+      for (int j = a.ooff[u] + 2; j < a.ooff[u + 1]; j++) cc_link(u, a.onbr[j], a.comp, a.err);
+      if (a.ioff)
+        for (int j = a.ioff[u]; j < a.ioff[u + 1]; j++) cc_link(u, a.inbr[j], a.comp, a.err);
+    }
+    __syncwarp();
+  }
+}
+
+// One cooperative launch does a whole run, with a grid barrier between the
+// phases (separate launches: 312 us at Kronecker 2^23, 70 us on 1,000
+// vertices; 259 and 34 this way).
+__global__ void __launch_bounds__(kThreads, kCtasPerSm) cc_kernel(const CcArgs a) {
+  __shared__ int s_min[kThreads / 32];
+  __shared__ int s_ok;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
+  const int64_t gtid = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  const int giant = 0;  // the root of row 0's component
+  unsigned round = 0;
+  auto barrier = [&] {
+    const bool ok = grid_barrier(a.barrier, ++round, &s_ok);
+    if (!ok && threadIdx.x == 0) *a.err = 2;
+    return ok;
+  };
+  // roots of the rows [0, active) are rows of [0, active)
+  for (int64_t v = gtid; v < a.active; v += stride) {
+    a.comp[v] = static_cast<int>(v);
+    a.root_min[v] = INT_MAX;
+  }
+  if (!barrier()) return;
+  for (int r = 0; r < 2; r++) {  // neighbor_rounds of src/cc.cc:92
+    if (r == 0) sample_first(a, gtid, stride);
+    else sample_second(a, gtid, stride);
+    if (!barrier()) return;
+    for (int64_t v = gtid; v < a.active; v += stride)
+      compress_one(static_cast<int>(v), a.comp, a.err);
+    if (!barrier()) return;
+  }
+  link_rest(a, giant);
+  if (!barrier()) return;
+  // The last compress, fused with the ids mapped back: every vertex chases
+  // to its root and offers its original id to the root's minimum.  Members
+  // of the component of row 0 (the largest one; half the graph on Kronecker
+  // inputs) are reduced per thread and per block first, so its root takes
+  // one atomic per block instead of one per vertex.
+  int local = INT_MAX;
+  for (int64_t v = gtid; v < a.active; v += stride) {
+    const int c = compress_one(static_cast<int>(v), a.comp, a.err);
+    if (c == giant) local = min(local, a.perm[v]);
+    else atomicMin(a.root_min + c, a.perm[v]);
   }
   local = static_cast<int>(__reduce_min_sync(0xffffffffu, static_cast<unsigned>(local)));
   if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = local;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    int m = INT_MAX;
-    for (int w = 0; w < (blockDim.x >> 5); w++) m = min(m, s_min[w]);
-    if (m != INT_MAX) atomicMin(root_min + giant, m);
+  if (threadIdx.x < 32) {
+    const int m = static_cast<int>(
+        __reduce_min_sync(0xffffffffu, static_cast<unsigned>(s_min[threadIdx.x])));
+    if (threadIdx.x == 0 && m != INT_MAX) atomicMin(a.root_min + giant, m);
   }
-}
-
-// Label of every original id o (a gather, so the writes are coalesced):
-// rows [active, n) have no edges and are their own components.
-__global__ void cc_label_kernel(int32_t n, int32_t active, const int *comp,
-                                const int32_t *__restrict__ inv, const int *root_min,
-                                int32_t *out_old) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t o = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; o < n; o += stride) {
-    const int v = inv[o];
-    // comp and root_min are final here (read-only path)
-    out_old[o] = v < active ? __ldg(root_min + __ldg(comp + v)) : static_cast<int32_t>(o);
+  if (!barrier()) return;
+  // Label of every original id o (a gather, so the writes are coalesced):
+  // rows [active, n) have no edges and are their own components.
+  for (int64_t o = gtid; o < a.n; o += stride) {
+    const int v = a.inv[o];
+    a.out_old[o] = v < a.active ? a.root_min[a.comp[v]] : static_cast<int32_t>(o);
   }
-}
-
-__global__ void fill_kernel(int32_t n, int value, int *a) {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
-    a[i] = value;
-}
-
-unsigned CcGrid(int64_t items) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, sms * 16)));
+  leave_grid(a.barrier);
 }
 
 }  // namespace
 
 void FreeCcScratch(CcScratch *c) {
-  for (int *p : {c->comp, c->root_min, c->err})
+  for (void *p : {static_cast<void *>(c->comp), static_cast<void *>(c->root_min),
+                  static_cast<void *>(c->second), c->barrier})
     if (p) cudaFree(p);
-  c->comp = c->root_min = c->err = nullptr;
-  c->cap = 0;
+  if (c->err) cudaFreeHost(c->err);
+  *c = CcScratch();
 }
 
 cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_t s,
                                 int32_t *out_old, std::string *err) {
   const int32_t n = static_cast<int32_t>(g.n);
-  // out-CSR in new ids: the shared CSR of an undirected graph, the
-  // renumbered out-CSR of a directed one
-  const int32_t *ooff = g.directed ? g.orowoff : g.rowoff;
-  const int32_t *onbr = g.directed ? g.ocol : g.col;
   cudaError_t e = cudaSuccess;
   if (!cs.comp || cs.cap < n) {
     FreeCcScratch(&cs);
-    e = cudaMalloc(&cs.comp, sizeof(int) * std::max<int64_t>(n, 1));
-    if (e == cudaSuccess) e = cudaMalloc(&cs.root_min, sizeof(int) * std::max<int64_t>(n, 1));
-    if (e == cudaSuccess) e = cudaMalloc(&cs.err, sizeof(int));
+    const size_t bytes = sizeof(int) * std::max<int64_t>(n, 1);
+    e = cudaMalloc(&cs.comp, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&cs.root_min, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&cs.second, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&cs.barrier, sizeof(GridBarrier));
+    if (e == cudaSuccess) e = cudaMemsetAsync(cs.barrier, 0, sizeof(GridBarrier), s);
+    if (e == cudaSuccess)
+      e = cudaHostAlloc(reinterpret_cast<void **>(&cs.err), sizeof(int),
+                        cudaHostAllocMapped | cudaHostAllocPortable);
     if (e != cudaSuccess) {
       FreeCcScratch(&cs);
       *err = std::string("connected components: ") + cudaGetErrorString(e);
@@ -275,49 +285,43 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
     }
     cs.cap = n;
   }
-  int *comp = cs.comp, *root_min = cs.root_min, *derr = cs.err;
-  e = cudaMemsetAsync(derr, 0, sizeof(int), s);
-  const unsigned grid = CcGrid(n);
-  const int kRounds = 2;  // neighbor_rounds of src/cc.cc:92
+  CcArgs a;
+  a.n = n;
   // Rows without in-neighbours form the tail of the mirror; in an undirected
   // graph they have no edges at all, so no link ever touches them and they
   // stay their own components: the link and compress passes stop before them.
-  const int32_t active = g.directed ? n : static_cast<int32_t>(g.bin_row_start[kBinZero]);
+  a.active = g.directed ? n : static_cast<int32_t>(g.bin_row_start[kBinZero]);
   // rows of at least 32 entries (the front of the mirror) take a warp each
-  const int32_t long_rows = std::min<int32_t>(active, static_cast<int32_t>(g.bin_row_start[4]));
-  if (e == cudaSuccess) {
-    cc_init_kernel<<<CcGrid(active), 256, 0, s>>>(active, comp);
-    for (int r = 0; r < kRounds; r++) {
-      cc_sample_kernel<<<CcGrid(active), 256, 0, s>>>(active, ooff, onbr, r, comp, derr);
-      cc_compress_kernel<<<CcGrid(active), 256, 0, s>>>(active, comp, derr);
-    }
-    e = cudaGetLastError();
-  }
-  const int giant = 0;  // the root, and label, of row 0's component
-  if (e == cudaSuccess) {
-    const int32_t *ioff = g.directed ? g.rowoff : nullptr;
-    const int32_t *inbr = g.directed ? g.col : nullptr;
-    if (long_rows > 0)
-      cc_finish_warp_kernel<<<CcGrid(static_cast<int64_t>(long_rows) * 32), 256, 0, s>>>(
-          0, long_rows, ooff, onbr, ioff, inbr, kRounds, giant, comp, derr);
-    if (active > long_rows)
-      cc_finish_thread_kernel<<<CcGrid(active - long_rows), 256, 0, s>>>(
-          long_rows, active, ooff, onbr, ioff, inbr, kRounds, giant, comp, derr);
-    // roots of the rows [0, active) are rows of [0, active)
-    fill_kernel<<<CcGrid(active), 256, 0, s>>>(active, INT_MAX, root_min);
-    cc_compress_min_kernel<<<CcGrid(active), 256, 0, s>>>(active, comp, g.perm, root_min, derr);
-    cc_label_kernel<<<grid, 256, 0, s>>>(n, active, comp, g.inv, root_min, out_old);
-    e = cudaGetLastError();
-  }
-  int herr = 0;
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, s);
+  a.long_rows = std::min<int32_t>(a.active, static_cast<int32_t>(g.bin_row_start[4]));
+  // out-CSR in new ids: the shared CSR of an undirected graph, the
+  // renumbered out-CSR of a directed one
+  a.ooff = g.directed ? g.orowoff : g.rowoff;
+  a.onbr = g.directed ? g.ocol : g.col;
+  a.ioff = g.directed ? g.rowoff : nullptr;
+  a.inbr = g.directed ? g.col : nullptr;
+  a.perm = g.perm;
+  a.inv = g.inv;
+  a.comp = cs.comp;
+  a.root_min = cs.root_min;
+  a.second = cs.second;
+  a.out_old = out_old;
+  a.barrier = static_cast<GridBarrier *>(cs.barrier);
+  a.err = cs.err;
+  *cs.err = 0;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int grid = std::max(1, std::min((n + kThreads - 1) / kThreads, sms * kCtasPerSm));
+  e = LaunchGrid(reinterpret_cast<const void *>(cc_kernel), grid, kThreads, &a, 0, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     *err = std::string("connected components: ") + cudaGetErrorString(e);
     return e;
   }
-  if (herr) {
-    *err = "connected components: link or compress exceeded its iteration limit";
+  if (*cs.err) {
+    *err = *cs.err == 1 ? "connected components: link or compress exceeded its iteration limit"
+                        : "connected components: a grid barrier ran out of its wait";
+    cudaMemsetAsync(cs.barrier, 0, sizeof(GridBarrier), s);
     return cudaErrorUnknown;
   }
   return cudaSuccess;

@@ -222,7 +222,10 @@ void WidenOffsets(int64_t n1, const int32_t *off32, int64_t *off64, cudaStream_t
 // Connected components of the uploaded graph (cc.cu): out_old[v] = the
 // smallest original vertex id of v's component (device buffer, n entries).
 struct CcScratch {
-  int *comp = nullptr, *root_min = nullptr, *err = nullptr;
+  int *comp = nullptr, *root_min = nullptr;
+  int *second = nullptr;     // second out-neighbour of each vertex, -1 for none
+  void *barrier = nullptr;   // GridBarrier
+  int *err = nullptr;        // page-locked
   int64_t cap = 0;
 };
 void FreeCcScratch(CcScratch *c);

@@ -1249,8 +1249,9 @@ int pr_gpu_verify(pr_gpu_t *h, const float *scores, float damping, double *error
     PR_CHECK(h, prgpu::SumInOrder(n, h->sc.outbuf, h->ver, error_out, h->stream));
     return PR_GPU_OK;
   }
-  std::vector<float> resid(n);
-  rc = CopyToHost(h, resid.data(), h->sc.outbuf, sizeof(float) * n);
+  std::unique_ptr<float[]> resid(new (std::nothrow) float[n]);
+  if (!resid) return SetErr(h, PR_GPU_ENOMEM, "host buffer for the residuals");
+  rc = CopyToHost(h, resid.get(), h->sc.outbuf, sizeof(float) * n);
   if (rc) return rc;
   double error = 0;
   for (int64_t v = 0; v < n; v++) error += static_cast<double>(resid[v]);
