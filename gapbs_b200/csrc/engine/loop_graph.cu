@@ -74,8 +74,13 @@ cudaError_t LoopGraph::Build(const SweepKernel *ks, int nk, LoopCtl *ctl, int ma
   std::vector<Cached> body;
   if (e == cudaSuccess) {
     cudaGraph_t bg = cp.conditional.phGraph_out[0];
-    cudaGraphNode_t prev = nullptr;
+    // nodes that the next one waits for, and those that the last one waited for
+    std::vector<cudaGraphNode_t> deps, before;
     for (int i = 0; i < nk && e == cudaSuccess; i++) {
+      if (!ks[i].beside_previous) {
+        before = deps;
+        deps.clear();
+      }
       Cached c{ks[i].fn, ks[i].grid, ks[i].block, ks[i].smem,
                std::vector<unsigned char>(static_cast<const unsigned char *>(ks[i].args),
                                           static_cast<const unsigned char *>(ks[i].args) +
@@ -88,8 +93,8 @@ cudaError_t LoopGraph::Build(const SweepKernel *ks, int nk, LoopCtl *ctl, int ma
       kp.sharedMemBytes = static_cast<unsigned>(c.smem);
       kp.kernelParams = params;
       cudaGraphNode_t node = nullptr;
-      e = cudaGraphAddKernelNode(&node, bg, prev ? &prev : nullptr, prev ? 1 : 0, &kp);
-      prev = node;
+      e = cudaGraphAddKernelNode(&node, bg, before.data(), before.size(), &kp);
+      deps.push_back(node);
       body.push_back(std::move(c));
     }
     if (e == cudaSuccess) {
@@ -103,7 +108,7 @@ cudaError_t LoopGraph::Build(const SweepKernel *ks, int nk, LoopCtl *ctl, int ma
       dp.blockDim = dim3(32);
       dp.kernelParams = decide_params;
       cudaGraphNode_t decide_node = nullptr;
-      e = cudaGraphAddKernelNode(&decide_node, bg, prev ? &prev : nullptr, prev ? 1 : 0, &dp);
+      e = cudaGraphAddKernelNode(&decide_node, bg, deps.data(), deps.size(), &dp);
     }
   }
   if (e == cudaSuccess) e = cudaGraphInstantiate(&exec_, g, 0);

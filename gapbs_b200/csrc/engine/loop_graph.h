@@ -38,6 +38,7 @@ struct SweepKernel {
   size_t smem = 0;
   const void *args = nullptr;
   size_t args_size = 0;
+  bool beside_previous = false;  // may run at the same time as the kernel before it
 };
 
 class LoopGraph {

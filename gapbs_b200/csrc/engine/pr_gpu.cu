@@ -626,6 +626,7 @@ int SolveSingle(pr_gpu_t *h, int max_iters, double epsilon, float damping,
       body[i].smem = i < 2 ? prgpu::SliceSmemBytes(sb) : prgpu::BinSmemBytes(sb);
       body[i].args = &ba;
       body[i].args_size = sizeof(ba);
+      body[i].beside_previous = i == 1;
     }
   }
   PR_CHECK(h, cudaEventRecord(h->ev[1], s));
