@@ -31,8 +31,8 @@
 //     slice): per pair its position in its bin's block; row u's pairs are
 //     idx[rowq[u] .. rowq[u + 1]).
 //  6. Phase-1 work is cut, per launch (flat runs / the others), into
-//     segments: pieces of one run of about 1 / (6 x CTAs) of the launch's
-//     estimated instruction count; consecutive segments of one slice are
+//     segments: pieces of one run of about 1 / (UnitsPerCta x CTAs) of the
+//     launch's estimated instruction count; consecutive segments of one slice are
 //     joined into units up to that size, so that short runs share one load
 //     of their slice; CTAs take units in order from a counter.
 #include <cuda_runtime.h>
@@ -592,6 +592,19 @@ struct CubTemp {
   }
 };
 
+// Units a CTA takes of a phase-1 launch.  A unit costs a load of its slice
+// (192 KB, about 3 us) beside its work, and small units even out the end of
+// the launch.  The two launches run beside each other, so the second one's
+// CTAs fill the end of the first: one unit each will do for it.  The first
+// gets the more the larger the graph, whose units then have work for a load.
+// Kronecker graphs, us a solve with 6 units each / 2 and 1 / 4 and 1 / 10 and
+// 1: 3 M vertices (33 slices) 1310 / 1030 / 1091 / 1273, 2^22 (49) 1542 / 1242
+// / 1286 / 1458, 2^23 (94) 2588 / 2340 / 2330 / 2509, 2^24 (181) 5006 / 4988 /
+// 4844 / 4846, 2^25 (347) 10396 / 10923 / 10595 / 10215.
+double UnitsPerCta(bool flat, int64_t nslices) {
+  return flat ? std::min(10.0, std::max(1.5, static_cast<double>(nslices) / 36.0)) : 1.0;
+}
+
 }  // namespace
 
 void FreeSliceBlocks(SliceBlocks *sb) {
@@ -890,8 +903,8 @@ cudaError_t BuildSliceBlocks(const DeviceGraph &g, int slice_verts, int bin_word
   bin_table_kernel<<<Blocks(nbins, T), T, 0, s>>>(nbins, bin_row0, pq, sb->bin);
   SB_TRY(cudaGetLastError());
 
-  // 6. phase-1 work: each run cut into segments of about 1 / (6 G) of its
-  //    launch's estimated work; consecutive segments of one slice joined
+  // 6. phase-1 work: each run cut into segments of about 1 / (UnitsPerCta G)
+  //    of its launch's estimated work; consecutive segments of one slice joined
   //    into units up to that size (so short runs share one slice load);
   //    CTAs take units from a counter
   const int G = sms;
@@ -908,7 +921,7 @@ cudaError_t BuildSliceBlocks(const DeviceGraph &g, int slice_verts, int bin_word
     for (int64_t r = 0; r < nruns; r++)
       if (FlatShape(rtab[r].w) == (flat != 0))
         total += static_cast<double>(GroupCost(rtab[r].w, flat)) * (rgb[r + 1] - rgb[r]);
-    const double target = std::max(1.0, total / (6.0 * G));
+    const double target = std::max(1.0, total / (UnitsPerCta(flat != 0, nslices) * G));
     double unit_cost = 0;
     for (int64_t r = 0; r < nruns; r++) {
       if (FlatShape(rtab[r].w) != (flat != 0)) continue;
