@@ -224,13 +224,14 @@ __global__ void __launch_bounds__(kThreads, 1) resident_solve_kernel(const Resid
   const int lane32 = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const unsigned tile_sm = static_cast<unsigned>(__cvta_generic_to_shared(sm + 4));
   unsigned round = 0;
-  const int gthreads = gridDim.x * kThreads;
-  const int gtid = blockIdx.x * kThreads + threadIdx.x;
+  const int64_t gthreads = static_cast<int64_t>(gridDim.x) * kThreads;
+  const int64_t gtid = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
 
   // ---- init: s_0 = t (1/N), base = (1-d) t, contrib = s_0 / out_degree;
   // adjoint: lambda_0 = base = w, and ||w||_1 for the stop rule
   double norm = 0;
-  for (int u = gtid; u < a.n; u += gthreads) {
+  for (int64_t i = gtid; i < a.n; i += gthreads) {
+    const int u = static_cast<int>(i);
     const float t = a.in_old ? a.in_old[a.perm[u]] : a.init_scalar;
     a.score[u] = t;
     if (KIND == kKindAdjoint) {
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_solve_kernel(const Resid
     a.res->sweep_ns = static_cast<double>(global_ns() - t_begin);
   }
   if (a.out_old) {
-    for (int v = gtid; v < a.n; v += gthreads) {
+    for (int64_t v = gtid; v < a.n; v += gthreads) {
       const float x = __ldcg(a.score + a.inv[v]);
       a.out_old[v] = KIND == kKindAdjoint ? __fmul_rn(a.one_minus_d, x) : x;
     }

@@ -119,8 +119,8 @@ int pr_gpu_download_csr(pr_gpu_t *h, int64_t *out_off, int32_t *out_nbr);
  * (src/bfs.cc:118-160): kind "i" (init), "td" (top-down; count = next
  * frontier size), "e" (queue to bitmap), "bu" (bottom-up; count = vertices
  * found), "c" (bitmap to queue); count -1 where the reference prints none.
- * seconds: the step's duration measured on the device (the steps run as
- * one CUDA graph, so no host clock sees them one by one). */
+ * seconds: the step's duration measured on the device (a search is one
+ * launch, so no host clock sees the steps one by one). */
 typedef struct pr_gpu_bfs_step {
   char kind[4];
   int64_t count;

@@ -108,3 +108,26 @@ def test_long_trace(engine):
     assert int(r.sweeps[0]) == 5000 and r.err_trace.shape == (5000, 1)
     short = engine.run(50, 0.0)
     assert np.array_equal(r.err_trace[:50], short.err_trace)
+
+
+def test_large_uniform_graph_keeps_sweep_launches(engine):
+    """Over 2^23 vertices without hubs: the sweep kernels in a loop graph, plain
+    and adjoint, at a fixed number of sweeps."""
+    n = (1 << 23) + 5
+    rng = np.random.default_rng(8)
+    u, v = rng.integers(0, n, (2, 2 * n), dtype=np.int32)
+    u[0] = n - 1
+    g = Graph.from_edges(u, v, symmetrize=True)
+    engine.upload(g)
+    res = engine.run(4, 0.0)
+    s64, _, _ = oracle.pr_pull_f64(g, 4, 0.0)
+    assert int(res.sweeps[0]) == 4
+    assert np.all(np.abs(res.scores - s64) <= 2e-5 * np.abs(s64) + 1e-10)
+    w = rng.normal(size=g.num_nodes).astype(np.float32)
+    gt, ge, sweeps = engine.adjoint(w, res.scores, max_iters=5, epsilon=0.0)
+    assert sweeps == 5
+    _, gt64, gw64, _ = oracle.ppr_adjoint_f64(g.num_nodes, g.out_offsets, g.out_neighbors, w,
+                                              res.scores.astype(np.float64), max_iters=5,
+                                              epsilon=0.0)
+    assert np.linalg.norm(gt - gt64) <= 1e-4 * np.linalg.norm(gt64)
+    assert np.linalg.norm(ge - gw64) <= 1e-3 * np.linalg.norm(gw64)
