@@ -256,9 +256,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cc_kernel(const CcArgs a
 }  // namespace
 
 void FreeCcScratch(CcScratch *c) {
-  for (void *p : {static_cast<void *>(c->comp), static_cast<void *>(c->root_min),
-                  static_cast<void *>(c->second), c->barrier})
-    if (p) cudaFree(p);
+  if (c->mem) cudaFree(c->mem);
   if (c->err) cudaFreeHost(c->err);
   *c = CcScratch();
 }
@@ -269,12 +267,10 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
   cudaError_t e = cudaSuccess;
   if (!cs.comp || cs.cap < n) {
     FreeCcScratch(&cs);
-    const size_t bytes = sizeof(int) * std::max<int64_t>(n, 1);
-    e = cudaMalloc(&cs.comp, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&cs.root_min, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&cs.second, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&cs.barrier, sizeof(GridBarrier));
-    if (e == cudaSuccess) e = cudaMemsetAsync(cs.barrier, 0, sizeof(GridBarrier), s);
+    // one block: the barrier, then the three arrays
+    const int64_t cells = (static_cast<int64_t>(n) + 63) & ~int64_t(63);
+    e = cudaMalloc(&cs.mem, 256 + 3 * sizeof(int) * cells);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cs.mem, 0, sizeof(GridBarrier), s);
     if (e == cudaSuccess)
       e = cudaHostAlloc(reinterpret_cast<void **>(&cs.err), sizeof(int),
                         cudaHostAllocMapped | cudaHostAllocPortable);
@@ -283,6 +279,9 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
       *err = std::string("connected components: ") + cudaGetErrorString(e);
       return e;
     }
+    cs.comp = reinterpret_cast<int *>(static_cast<char *>(cs.mem) + 256);
+    cs.root_min = cs.comp + cells;
+    cs.second = cs.root_min + cells;
     cs.cap = n;
   }
   CcArgs a;
@@ -305,7 +304,7 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
   a.root_min = cs.root_min;
   a.second = cs.second;
   a.out_old = out_old;
-  a.barrier = static_cast<GridBarrier *>(cs.barrier);
+  a.barrier = static_cast<GridBarrier *>(cs.mem);
   a.err = cs.err;
   *cs.err = 0;
   int dev = 0, sms = 148;
@@ -321,7 +320,7 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
   if (*cs.err) {
     *err = *cs.err == 1 ? "connected components: link or compress exceeded its iteration limit"
                         : "connected components: a grid barrier ran out of its wait";
-    cudaMemsetAsync(cs.barrier, 0, sizeof(GridBarrier), s);
+    cudaMemsetAsync(cs.mem, 0, sizeof(GridBarrier), s);
     return cudaErrorUnknown;
   }
   return cudaSuccess;

@@ -224,7 +224,7 @@ void WidenOffsets(int64_t n1, const int32_t *off32, int64_t *off64, cudaStream_t
 struct CcScratch {
   int *comp = nullptr, *root_min = nullptr;
   int *second = nullptr;     // second out-neighbour of each vertex, -1 for none
-  void *barrier = nullptr;   // GridBarrier
+  void *mem = nullptr;       // holds a GridBarrier and the arrays
   int *err = nullptr;        // page-locked
   int64_t cap = 0;
 };
