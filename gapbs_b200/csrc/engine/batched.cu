@@ -358,6 +358,7 @@ __device__ __forceinline__ void sweep_rows(const BatchArgs &a, int it, const flo
   // ticket) adds the row's partials by a fixed tree and updates the row
   if (gw < a.nseg) {
     __threadfence();
+    __syncwarp();  // lane 0's ticket follows every lane's partial and fence
     for (int k = gw; k < a.nseg; k += nw) {
       const int4 sg = a.seg[k];
       const int u = sg.x;

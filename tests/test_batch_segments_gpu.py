@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from gapbs_b200 import PageRankEngine
+from gapbs_b200.graph import Graph
 from conftest import gpu_available
 from test_ppr_gpu import check_columns
 from test_resident_gpu import hub_graph
@@ -47,3 +48,24 @@ def test_row_lengths_and_first_sweep(engine, k):
     check_columns(g, sparse, a)
     b = engine.run(20, 1e-4, teleport=sparse)
     assert np.array_equal(a.scores.view(np.uint32), b.scores.view(np.uint32))
+
+
+@pytest.mark.parametrize("k", [12, 64])
+def test_warps_with_segments_only(engine, k):
+    """Every row is cut into segments and no warp has ordinary rows between a
+    partial and its ticket: the last segment's warp must see all columns of
+    the other warps' partials, in every sweep of repeated solves."""
+    rng = np.random.default_rng(17)
+    n = 400
+    u, v = np.divmod(rng.choice(n * n, 120000, replace=False), n)
+    g = Graph.from_edges(u.astype(np.int32), v.astype(np.int32))
+    assert np.diff(g.in_offsets).min() >= 256
+    engine.upload(g)
+    T = rng.random((n, k)).astype(np.float32)
+    T /= T.sum(axis=0)
+    first = engine.run(20, 1e-6, teleport=T)
+    check_columns(g, T, first, eps=1e-6)
+    for _ in range(20):
+        again = engine.run(20, 1e-6, teleport=T)
+        assert np.array_equal(first.scores.view(np.uint32), again.scores.view(np.uint32))
+        assert np.array_equal(first.err_trace, again.err_trace)
