@@ -133,15 +133,16 @@ __device__ __forceinline__ float4 row_accumulate(const BatchArgs &a, const float
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   int idx_next = 0;
   float w_next = 0.f;
-  if (s + lane < e) {
+  const unsigned end = e;  // j0 + 32 + lane may pass 2^31
+  if (static_cast<unsigned>(s) + lane < end) {
     idx_next = ld_stream_s32(a.col + s + lane, ps);
     if (W) w_next = ld_stream_f32(a.win + s + lane, ps);
   }
-  for (int j0 = s; j0 < e; j0 += 32) {
-    const int cnt = min(32, e - j0);
+  for (unsigned j0 = s; j0 < end; j0 += 32) {
+    const int cnt = min(32u, end - j0);
     int idx = idx_next;
     const float w = w_next;
-    if (j0 + 32 + lane < e) {  // fetched while this round's rows are gathered
+    if (j0 + 32 + lane < end) {  // fetched while this round's rows are gathered
       idx_next = ld_stream_s32(a.col + j0 + 32 + lane, ps);
       if (W) w_next = ld_stream_f32(a.win + j0 + 32 + lane, ps);
     }
@@ -362,7 +363,9 @@ __device__ __forceinline__ void sweep_rows(const BatchArgs &a, int it, const flo
     for (int k = gw; k < a.nseg; k += nw) {
       const int4 sg = a.seg[k];
       const int u = sg.x;
-      const int nseg = (a.rowoff[u + 1] - a.rowoff[u] + a.segment - 1) / a.segment;
+      const int nseg = static_cast<int>(
+          (static_cast<unsigned>(a.rowoff[u + 1] - a.rowoff[u]) + a.segment - 1u) /
+          static_cast<unsigned>(a.segment));
       int last = 0;
       if (lane == 0) last = atomicAdd(a.ticket + sg.y, 1u) == static_cast<unsigned>(nseg - 1);
       if (!__shfl_sync(0xffffffffu, last, 0)) continue;

@@ -88,7 +88,8 @@ __global__ void rowid_kernel(int32_t ndst, const int32_t *__restrict__ rowoff, i
   const int lane = threadIdx.x & 31;
   if (warp >= ndst) return;
   const int32_t u = static_cast<int32_t>(warp);
-  for (int32_t e = rowoff[u] + lane; e < rowoff[u + 1]; e += 32) rowid[e] = u;
+  const uint32_t end = rowoff[u + 1];  // e + 32 may pass 2^31
+  for (uint32_t e = rowoff[u] + lane; e < end; e += 32) rowid[e] = u;
 }
 
 __global__ void slice_key_kernel(int64_t m, const int32_t *__restrict__ col, int32_t slice_verts,

@@ -177,11 +177,14 @@ __device__ __forceinline__ void link_rest(const CcArgs &a, int giant) {
     while (together) {
       const int w = static_cast<int>(b << 5) + __ffs(together) - 1;
       together &= together - 1;
-      for (int j = a.ooff[w] + 2 + lane; j < a.ooff[w + 1]; j += 32)
+      const unsigned oe = a.ooff[w + 1];  // j + 32 may pass 2^31
+      for (unsigned j = a.ooff[w] + 2u + lane; j < oe; j += 32)
         cc_link(w, a.onbr[j], a.comp, a.err);
-      if (a.ioff)
-        for (int j = a.ioff[w] + lane; j < a.ioff[w + 1]; j += 32)
+      if (a.ioff) {
+        const unsigned ie = a.ioff[w + 1];
+        for (unsigned j = a.ioff[w] + static_cast<unsigned>(lane); j < ie; j += 32)
           cc_link(w, a.inbr[j], a.comp, a.err);
+      }
       __syncwarp();
     }
     if (left && u >= a.long_rows) {
@@ -310,7 +313,8 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int grid = std::max(1, std::min((n + kThreads - 1) / kThreads, sms * kCtasPerSm));
+  const int grid = static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>((g.n + kThreads - 1) / kThreads, sms * kCtasPerSm)));
   e = LaunchGrid(reinterpret_cast<const void *>(cc_kernel), grid, kThreads, &a, 0, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {

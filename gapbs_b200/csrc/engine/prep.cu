@@ -111,9 +111,9 @@ __global__ void renumber_rows_kernel(int64_t n, const int32_t *__restrict__ perm
   const int lane = threadIdx.x & 31;
   if (warp >= n) return;
   const int32_t v = perm[warp];
-  const int32_t s = src_off[v], len = src_off[v + 1] - s;
-  const int32_t d = dst_off[warp];
-  for (int32_t j = lane; j < len; j += 32) {
+  const uint32_t s = src_off[v], len = src_off[v + 1] - s;
+  const uint32_t d = dst_off[warp];
+  for (uint32_t j = lane; j < len; j += 32) {
     const int32_t x = src_nbr[s + j];
     dst_nbr[d + j] = translate ? translate[x] : x;
   }
@@ -145,11 +145,11 @@ struct RowWeightArgs {
 template <int T>
 __device__ __forceinline__ void row_weights(const RowWeightArgs &a, int p, int t, double *sred) {
   const int32_t v = a.order ? a.order[p] : p;
-  const int32_t s = a.orig_off[a.perm[v]], d = a.orow[v];
-  const int32_t len = a.orow[v + 1] - d;
+  const uint32_t s = a.orig_off[a.perm[v]], d = a.orow[v];
+  const uint32_t len = a.orow[v + 1] - d;
   double acc = 0;
 #pragma unroll 4
-  for (int32_t j = t; j < len; j += T) {
+  for (uint32_t j = t; j < len; j += T) {
     const float x = a.w[s + j];
     a.wout[d + j] = x;
     acc += x;
@@ -184,9 +184,9 @@ __global__ void in_weight_kernel(int64_t n, const int32_t *__restrict__ perm,
   const int lane = threadIdx.x & 31;
   if (warp >= n) return;
   const int32_t v = perm[warp];
-  const int32_t s = in_off[v], len = in_off[v + 1] - s;
-  const int32_t d = rowoff[warp];
-  for (int32_t j = lane; j < len; j += 32) {
+  const uint32_t s = in_off[v], len = in_off[v + 1] - s;
+  const uint32_t d = rowoff[warp];
+  for (uint32_t j = lane; j < len; j += 32) {
     const int32_t x = in_nbr[s + j];
     int32_t lo = out_off[x], hi = out_off[x + 1];
     while (lo < hi) {

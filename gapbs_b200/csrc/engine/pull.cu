@@ -160,8 +160,8 @@ __device__ __forceinline__ float warp_task(const PullArgs &a, const float *cin, 
                                            uint64_t pg, uint64_t pl) {
   constexpr int kRowsPerTask = 32 / G;
   const int lane = lane32 % G;
-  const int u = a.bin_row[bin] + task * kRowsPerTask + lane32 / G;
-  const bool valid = u < a.bin_row[bin + 1];
+  const unsigned u = static_cast<unsigned>(a.bin_row[bin]) + task * kRowsPerTask + lane32 / G;
+  const bool valid = u < static_cast<unsigned>(a.bin_row[bin + 1]);
   int s = 0, e = 0;
   float old = 0.f;
   if (valid) {
@@ -189,7 +189,7 @@ __device__ __forceinline__ float hub_segment(const PullArgs &a, const float *cin
   const int nseg = a.seg_first[u + 1] - first;
   const int rs = a.rowoff[u], re = a.rowoff[u + 1];
   const int s = rs + (seg - first) * kSegEntries;
-  const int e = min(re, s + kSegEntries);
+  const int e = s + min(re - s, kSegEntries);  // s + kSegEntries may pass 2^31
   float acc = lane_partial<kSweepThreads, W>(a, cin, s, e, threadIdx.x, ps, pg);
   const float part = block_sum_f<kSweepThreads>(acc, sredf);
   if (threadIdx.x == 0) {
@@ -216,18 +216,18 @@ template <bool W, bool DIR, int KIND>
 __device__ __forceinline__ double zero_task(const PullArgs &a, float *cout, int task, int lane32,
                                            uint64_t ps, uint64_t pl) {
   constexpr int kRows = 32 * kZeroRowsPerThread;
-  const int row0 = a.bin_row[kBinZero] + task * kRows;
-  const int end = a.bin_row[kBinZero + 1];
+  const unsigned row0 = static_cast<unsigned>(a.bin_row[kBinZero]) + task * kRows;
+  const unsigned end = a.bin_row[kBinZero + 1];  // row0 + kRows may pass 2^31
   float old[kZeroRowsPerThread];
 #pragma unroll
   for (int i = 0; i < kZeroRowsPerThread; i++) {
-    const int u = row0 + i * 32 + lane32;
+    const unsigned u = row0 + i * 32 + lane32;
     old[i] = u < end ? ld_score(a.score + u, ps) : 0.f;
   }
   double err = 0.0;
 #pragma unroll
   for (int i = 0; i < kZeroRowsPerThread; i++) {
-    const int u = row0 + i * 32 + lane32;
+    const unsigned u = row0 + i * 32 + lane32;
     if (u < end) {
       const float base = KIND != kKindPlain ? a.base_vec[u] : a.base_scalar;
       const float nw = pr_update(base, a.damping, 0.f);
@@ -315,10 +315,10 @@ struct GradArgs {
 template <int T>
 __device__ __forceinline__ void edge_grad_row(const GradArgs &a, int p, int t, double *sred) {
   const int v = a.order ? a.order[p] : p;
-  const int s = a.orow[v], e = a.orow[v + 1];
+  const unsigned s = a.orow[v], e = a.orow[v + 1];  // j + T may pass 2^31
   double acc = 0;
 #pragma unroll 4
-  for (int j = s + t; j < e; j += T)
+  for (unsigned j = s + t; j < e; j += T)
     acc += static_cast<double>(a.wout ? a.wout[j] : 1.f) * a.lam[a.ocol[j]];
   if (T == 32) {
     acc = warp_sum_d(acc);
@@ -334,7 +334,7 @@ __device__ __forceinline__ void edge_grad_row(const GradArgs &a, int p, int t, d
   const double coef = static_cast<double>(a.damping) * a.s_old[pv] / S;
   const int64_t base = a.orig_off[pv];
 #pragma unroll 4
-  for (int j = s + t; j < e; j += T)
+  for (unsigned j = s + t; j < e; j += T)
     a.grad_ew[base + (j - s)] = static_cast<float>(coef * (a.lam[a.ocol[j]] - plam));
 }
 
@@ -374,7 +374,7 @@ cudaError_t LaunchAdjointGrads(const DeviceGraph &g, const float *lam_new, const
                          s>>>(a, nlong, end);
   }
   if (grad_t_old)
-    adjoint_teleport_grad_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, g.inv, lam_new, 1.0f - damping,
+    adjoint_teleport_grad_kernel<<<(static_cast<unsigned>(n) + 255u) / 256u, 256, 0, s>>>(n, g.inv, lam_new, 1.0f - damping,
                                                                  grad_t_old);
   return cudaGetLastError();
 }
@@ -402,8 +402,8 @@ __global__ void pull_init_kernel(int32_t n, const int32_t *__restrict__ rowoff,
                                  const float *__restrict__ tele_new, float init_scalar,
                                  float one_minus_d, float *score, float *contrib,
                                  float *base) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= n) return;
+  const unsigned u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= static_cast<unsigned>(n)) return;
   const float t = tele_new ? tele_new[u] : init_scalar;
   score[u] = t;
   if (tele_new) base[u] = __fmul_rn(one_minus_d, t);
@@ -475,7 +475,7 @@ cudaError_t LaunchPullInit(const DeviceGraph &g, Scratch &sc, const float *tele_
   const int n = static_cast<int>(g.n);
   if (n == 0) return cudaSuccess;
   const int threads = 256;
-  const int blocks = (n + threads - 1) / threads;
+  const unsigned blocks = (static_cast<unsigned>(n) + threads - 1) / threads;
   const float omd = 1.0f - damping;
   if (g.weighted)
     pull_init_kernel<true, false><<<blocks, threads, 0, s>>>(

@@ -97,15 +97,18 @@ __device__ __forceinline__ float denom(const ResidentArgs &a, int u, int s, int 
 }
 
 // One lane's share of a row: entries [s, e) in aligned four-entry chunks
-// c, c + step, ...
+// c, c + step, ...  A graph may have 2^31 - 9 entries, so the first entry of a
+// chunk past the row's end needs all 32 bits: unsigned.
 struct Share {
   int s, e, c;
+  __device__ __forceinline__ unsigned first() const { return static_cast<unsigned>(c) << 2; }
+  __device__ __forceinline__ bool more() const { return first() < static_cast<unsigned>(e); }
 };
 
 template <bool W>
 __device__ __forceinline__ void load_chunk(const ResidentArgs &a, const Share &x, int4 &q,
                                            float4 &w, uint64_t ps) {
-  if ((x.c << 2) >= x.e) return;
+  if (!x.more()) return;
   q = ld_stream_v4(reinterpret_cast<const int4 *>(a.col) + x.c, ps);
   if (W) w = ld_stream_v4f(reinterpret_cast<const float4 *>(a.win) + x.c, ps);
 }
@@ -115,9 +118,9 @@ template <bool W>
 __device__ __forceinline__ void add_chunk(float &acc, const Share &x, const int4 &q,
                                           const float4 &w, const float *cin, unsigned tile_sm,
                                           int tile, uint64_t pg) {
-  if ((x.c << 2) >= x.e) return;
+  if (!x.more()) return;
   const unsigned len = x.e - x.s;
-  const unsigned d = (x.c << 2) - x.s;  // wraps below the row's start
+  const unsigned d = x.first() - x.s;  // wraps below the row's start
   const float v0 = gather1(tile_sm, tile, cin, d < len ? q.x : -1, pg);
   const float v1 = gather1(tile_sm, tile, cin, d + 1 < len ? q.y : -1, pg);
   const float v2 = gather1(tile_sm, tile, cin, d + 2 < len ? q.z : -1, pg);
@@ -139,7 +142,7 @@ __device__ __forceinline__ void sum_shares(const ResidentArgs &a, Share x, Share
                                            const float *cin, unsigned tile_sm, uint64_t ps,
                                            uint64_t pg, float &acc_x, float &acc_y) {
   acc_x = acc_y = 0.f;
-  while ((x.c << 2) < x.e || (y.c << 2) < y.e) {
+  while (x.more() || y.more()) {
     int4 qx, qy;
     float4 wx, wy;
     load_chunk<W>(a, x, qx, wx, ps);
@@ -181,6 +184,7 @@ struct Task {
   int lg;
 };
 
+// Row positions past a bin's end (up to 511 of them) may pass 2^31: unsigned.
 __device__ __forceinline__ Task load_task(const ResidentArgs &a, int t, int ntasks, int lane32) {
   Task x{0, 0, 0, 0, 0, 0, 5};
   if (t >= min(ntasks, a.task_start[kBinZero])) return x;
@@ -196,14 +200,14 @@ __device__ __forceinline__ Task load_task(const ResidentArgs &a, int t, int ntas
   for (int i = 2; i < kBinZero; i++) bin += (t >= a.task_start[i]);
   x.lg = 6 - bin;  // 32, 16, 8, 4, 2, 1 lanes a row
   const int k = (t - a.task_start[bin]) << (bin > 1 ? 6 - x.lg : 0);
-  const int p = a.row_start[bin] + k + (lane32 >> x.lg);
-  const int end = a.row_start[bin + 1];
+  const unsigned p = static_cast<unsigned>(a.row_start[bin]) + k + (lane32 >> x.lg);
+  const unsigned end = a.row_start[bin + 1];
   if (p < end) {
     x.u = a.order ? a.order[p] : p;
     x.s = a.rowoff[x.u];
     x.e = a.rowoff[x.u + 1];
   }
-  const int p2 = p + (32 >> x.lg);
+  const unsigned p2 = p + (32 >> x.lg);
   if (bin > 1 && p2 < end) {
     x.u2 = a.order ? a.order[p2] : p2;
     x.s2 = a.rowoff[x.u2];
@@ -325,12 +329,12 @@ __global__ void __launch_bounds__(kThreads, 1) resident_solve_kernel(const Resid
     }
     // rows without entries: new = base
     for (; t < ntasks; t += nw + back, back = -back) {
-      const int p0 = a.row_start[kBinZero] +
-                     (t - a.task_start[kBinZero]) * (32 * kZeroRowsPerThread) + lane32;
+      const unsigned p0 = static_cast<unsigned>(a.row_start[kBinZero]) +
+                          (t - a.task_start[kBinZero]) * (32 * kZeroRowsPerThread) + lane32;
 #pragma unroll
       for (int i = 0; i < kZeroRowsPerThread; i++) {
-        const int p = p0 + 32 * i;
-        if (p < a.n) {
+        const unsigned p = p0 + 32 * i;
+        if (p < static_cast<unsigned>(a.n)) {
           const int u = a.order ? a.order[p] : p;
           err += finish_row<W, DIR, KIND>(a, cout, u, 0, 0, 0.f, __ldcg(a.score + u), ps, pl);
         }
@@ -344,7 +348,8 @@ __global__ void __launch_bounds__(kThreads, 1) resident_solve_kernel(const Resid
       for (int k = gw; k < a.task_start[1]; k += nw + back, back = -back) {
         const int4 sg = a.seg[k];
         const int rs = a.rowoff[sg.x], re = a.rowoff[sg.x + 1];
-        const int nseg = (re - rs + a.segment - 1) / a.segment;
+        const int nseg = static_cast<int>((static_cast<unsigned>(re - rs) + a.segment - 1u) /
+                                          static_cast<unsigned>(a.segment));
         int last = 0;
         if (lane32 == 0)
           last = atomicAdd(a.ticket + sg.y, 1u) == static_cast<unsigned>(nseg - 1);
@@ -430,8 +435,8 @@ __global__ void row_bounds_kernel(int32_t n, const int32_t *__restrict__ rowoff,
 
 __global__ void row_lengths_kernel(int32_t count, const int32_t *__restrict__ rowoff,
                                    int32_t *len) {
-  const int u = blockIdx.x * blockDim.x + threadIdx.x;
-  if (u < count) len[u] = rowoff[u + 1] - rowoff[u];
+  const unsigned u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u < static_cast<unsigned>(count)) len[u] = rowoff[u + 1] - rowoff[u];
 }
 
 // (row, first entry, end) of the rows at positions 0 .. count-1.
@@ -446,8 +451,8 @@ __global__ void long_rows_kernel(int32_t count, const int32_t *__restrict__ rowo
 }
 
 __global__ void iota_kernel(int32_t n, int32_t *ids) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) ids[i] = i;
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < static_cast<unsigned>(n)) ids[i] = static_cast<int32_t>(i);
 }
 
 // Positions 0 .. n-1 of rows by descending length (stable).
@@ -463,8 +468,9 @@ cudaError_t SortRows(int32_t n, const int32_t *rowoff, int32_t *order, cudaStrea
                                                   0, 32, s);
   if (e == cudaSuccess) e = cudaMalloc(&tmp, bytes);
   if (e == cudaSuccess) {
-    row_lengths_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, rowoff, len);
-    iota_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, ids);
+    const unsigned blocks = (static_cast<unsigned>(n) + 255u) / 256u;
+    row_lengths_kernel<<<blocks, 256, 0, s>>>(n, rowoff, len);
+    iota_kernel<<<blocks, 256, 0, s>>>(n, ids);
     e = cub::DeviceRadixSort::SortPairsDescending(tmp, bytes, len, len_sorted, ids, order, n, 0,
                                                   32, s);
   }
@@ -543,9 +549,11 @@ cudaError_t BuildRowTasks(int32_t n, const int32_t *rowoff, bool sorted, const R
   }
   std::vector<int4> seg;
   for (int32_t p = 0; p < nlong && e == cudaSuccess; p++) {
-    const int32_t first = static_cast<int32_t>(seg.size()), end = row[3 * p + 2];
-    for (int32_t b = row[3 * p + 1]; b < end; b += rc.segment)
-      seg.push_back(make_int4(row[3 * p], first, b, std::min(end, b + rc.segment)));
+    const int32_t first = static_cast<int32_t>(seg.size());
+    const int64_t end = row[3 * p + 2];  // b + segment may pass 2^31
+    for (int64_t b = row[3 * p + 1]; b < end; b += rc.segment)
+      seg.push_back(make_int4(row[3 * p], first, static_cast<int>(b),
+                              static_cast<int>(std::min(end, b + rc.segment))));
   }
   if (e == cudaSuccess && nlong) {
     e = cudaMalloc(&r->seg, sizeof(int4) * seg.size());

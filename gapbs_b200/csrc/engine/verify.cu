@@ -90,19 +90,19 @@ __device__ __forceinline__ void hub_row(const VerifyArgs &a, float (*buf)[kHubCh
   static_assert(kHubChunk % kFetchers == 0, "whole rounds of fetches");
   const int t = static_cast<int>(threadIdx.x) - 32;  // the first warp never waits for loads
   const int64_t u = blockIdx.x;
-  const int32_t lo = a.rowoff[u], hi = a.rowoff[u + 1];
+  const uint32_t lo = a.rowoff[u], hi = a.rowoff[u + 1];  // at + kHubChunk may pass 2^31
   float v[kPer];
-  auto fetch = [&](int32_t at) {
+  auto fetch = [&](uint32_t at) {
 #pragma unroll
     for (int i = 0; i < kPer; i++) {
-      const int32_t j = at + i * kFetchers + t;
+      const uint32_t j = at + i * kFetchers + t;
       v[i] = j < hi ? a.contrib[a.col[j]] : 0.f;
     }
   };
   if (t >= 0) fetch(lo);
   float sum = 0.f;
   int k = 0;
-  for (int32_t at = lo; at < hi; at += kHubChunk, k ^= 1) {
+  for (uint32_t at = lo; at < hi; at += kHubChunk, k ^= 1) {
     if (t >= 0) {
 #pragma unroll
       for (int i = 0; i < kPer; i++) buf[k][i * kFetchers + t] = v[i];
@@ -111,7 +111,7 @@ __device__ __forceinline__ void hub_row(const VerifyArgs &a, float (*buf)[kHubCh
     if (t >= 0) {
       if (at + kHubChunk < hi) fetch(at + kHubChunk);
     } else {
-      const int cnt = min(kHubChunk, hi - at);
+      const int cnt = min(static_cast<uint32_t>(kHubChunk), hi - at);
       const float4 *b4 = reinterpret_cast<const float4 *>(buf[k]);
       int j = 0;
 #pragma unroll 8
@@ -134,12 +134,12 @@ __device__ __forceinline__ void hub_row(const VerifyArgs &a, float (*buf)[kHubCh
 // a fifth of the instructions but waited for two loads every 8 rows of 32
 // entries: 2,900 us for the launch at Kronecker 2^22 against 756.)
 __device__ __forceinline__ void long_row(const VerifyArgs &a, int64_t u, int lane) {
-  const int32_t lo = a.rowoff[u], hi = a.rowoff[u + 1];
+  const uint32_t lo = a.rowoff[u], hi = a.rowoff[u + 1];  // j + 63 may pass 2^31
   float sum = 0.f;
   float c = lo + lane < hi ? a.contrib[a.col[lo + lane]] : 0.f;
-  for (int32_t j = lo; j < hi; j += 32) {
-    const int cnt = min(32, hi - j);
-    const int32_t jn = j + 32 + lane;
+  for (uint32_t j = lo; j < hi; j += 32) {
+    const int cnt = min(32u, hi - j);
+    const uint32_t jn = j + 32 + lane;
     const float cn = jn < hi ? a.contrib[a.col[jn]] : 0.f;
     if (cnt == 32) {
 #pragma unroll
