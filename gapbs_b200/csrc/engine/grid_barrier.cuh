@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include "barrier_count.h"
 #include "resident.h"
 
 namespace prgpu {
@@ -29,7 +30,7 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier *b, unsigned round, int
     atomicAdd(&b->arrived, 1u);
     const unsigned want = round * gridDim.x;
     unsigned polls = 0;
-    while (ld_acquire(&b->arrived) < want && ++polls < kMaxPolls) {
+    while (!arrivals_reached(ld_acquire(&b->arrived), want) && ++polls < kMaxPolls) {
     }
     *s_ok = polls < kMaxPolls;
     __threadfence();
