@@ -118,6 +118,7 @@ struct BfsArgs {
   int32_t *out_old;
   int64_t m;
   int32_t n, in_rows, source_old, alpha, beta;
+  unsigned max_polls;
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -460,7 +461,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) bfs_kernel(const BfsArgs
   const int64_t gtid = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
   unsigned round = 0;
   auto barrier = [&] {
-    const bool ok = grid_barrier(&a.ctl->barrier, ++round, &s_ok);
+    const bool ok = grid_barrier(&a.ctl->barrier, ++round, a.max_polls, &s_ok);
     if (!ok && threadIdx.x == 0) a.res->error = 2;
     return ok;
   };
@@ -565,7 +566,8 @@ void FreeBfsScratch(BfsScratch *b) {
   } while (0)
 
 cudaError_t BreadthFirstSearch(const DeviceGraph &g, BfsScratch &b, cudaStream_t s,
-                               int source_old, int alpha, int beta, int32_t *out_old,
+                               int source_old, int alpha, int beta, unsigned max_polls,
+                               int32_t *out_old,
                                std::vector<BfsStep> *steps, int64_t *nsteps,
                                std::string *err) {
   const int64_t n = g.n;
@@ -610,6 +612,7 @@ cudaError_t BreadthFirstSearch(const DeviceGraph &g, BfsScratch &b, cudaStream_t
   // can only be reached as the source)
   a.in_rows = static_cast<int32_t>(g.bin_row_start[kBinZero]);
   a.source_old = source_old;
+  a.max_polls = max_polls;
   a.alpha = alpha;
   a.beta = beta;
   int dev = 0, sms = 148;

@@ -106,6 +106,7 @@ struct CcArgs {
   int *comp, *root_min, *second;
   int32_t *out_old;
   GridBarrier *barrier;
+  unsigned max_polls;
   int *err;  // page-locked: 1 an iteration limit, 2 a barrier wait ran out
 };
 
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) cc_kernel(const CcArgs a
   const int giant = 0;  // the root of row 0's component
   unsigned round = 0;
   auto barrier = [&] {
-    const bool ok = grid_barrier(a.barrier, ++round, &s_ok);
+    const bool ok = grid_barrier(a.barrier, ++round, a.max_polls, &s_ok);
     if (!ok && threadIdx.x == 0) *a.err = 2;
     return ok;
   };
@@ -265,7 +266,7 @@ void FreeCcScratch(CcScratch *c) {
 }
 
 cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_t s,
-                                int32_t *out_old, std::string *err) {
+                                unsigned max_polls, int32_t *out_old, std::string *err) {
   const int32_t n = static_cast<int32_t>(g.n);
   cudaError_t e = cudaSuccess;
   if (!cs.comp || cs.cap < n) {
@@ -308,6 +309,7 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
   a.second = cs.second;
   a.out_old = out_old;
   a.barrier = static_cast<GridBarrier *>(cs.mem);
+  a.max_polls = max_polls;
   a.err = cs.err;
   *cs.err = 0;
   int dev = 0, sms = 148;

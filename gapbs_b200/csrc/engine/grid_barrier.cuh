@@ -9,9 +9,6 @@
 
 namespace prgpu {
 
-// polls of the barrier before a CTA gives up (about 10 s)
-constexpr unsigned kMaxPolls = 1u << 24;
-
 __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -19,10 +16,13 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
 }
 
 // Thread 0 of every CTA arrives and waits until all have arrived `round`
-// times (1, 2, ... over a launch); false when the wait ran out.  Called by
-// all threads; what any CTA wrote before it is visible after it to loads that
-// the compiler may not serve from the read-only path.
-__device__ __forceinline__ bool grid_barrier(GridBarrier *b, unsigned round, int *s_ok) {
+// times (1, 2, ... over a launch); false when the wait ran out after
+// max_polls polls.  Called by all threads; what any CTA wrote before it is
+// visible after it to loads that the compiler may not serve from the
+// read-only path.  A CTA that gives up must return: it arrives no more, so no
+// CTA passes the next round, and what one reads after this round is complete.
+__device__ __forceinline__ bool grid_barrier(GridBarrier *b, unsigned round, unsigned max_polls,
+                                             int *s_ok) {
   __syncthreads();
   if (gridDim.x == 1) return true;
   if (threadIdx.x == 0) {
@@ -30,9 +30,10 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier *b, unsigned round, int
     atomicAdd(&b->arrived, 1u);
     const unsigned want = round * gridDim.x;
     unsigned polls = 0;
-    while (!arrivals_reached(ld_acquire(&b->arrived), want) && ++polls < kMaxPolls) {
+    bool all;
+    while (!(all = arrivals_reached(ld_acquire(&b->arrived), want)) && polls++ < max_polls) {
     }
-    *s_ok = polls < kMaxPolls;
+    *s_ok = all;
     __threadfence();
   }
   __syncthreads();

@@ -253,10 +253,11 @@ void FreeBfsScratch(BfsScratch *b);
 // (nullable): the first steps with device-measured durations; *nsteps
 // (nullable): the number of steps, init included.
 cudaError_t BreadthFirstSearch(const DeviceGraph &g, BfsScratch &b, cudaStream_t s,
-                               int source_old, int alpha, int beta, int32_t *parent_old,
-                               std::vector<BfsStep> *steps, int64_t *nsteps, std::string *err);
+                               int source_old, int alpha, int beta, unsigned max_polls,
+                               int32_t *parent_old, std::vector<BfsStep> *steps,
+                               int64_t *nsteps, std::string *err);
 cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_t s,
-                                int32_t *out_old, std::string *err);
+                                unsigned max_polls, int32_t *out_old, std::string *err);
 // int64 CSR offsets -> int32, setting *bad for values outside [0, 2^31).
 void NarrowOffsets(int64_t count, const int64_t *wide, int32_t *narrow, int *bad, cudaStream_t s);
 

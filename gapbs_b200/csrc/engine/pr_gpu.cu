@@ -70,6 +70,7 @@ struct pr_gpu {
   prgpu::CcScratch cc;    // connected-components work arrays
   prgpu::BfsScratch bfs;  // breadth-first-search work arrays
   prgpu::VerifyScratch ver;
+  int64_t wait_polls = -1;  // pr_gpu_set_wait_limit
 };
 
 namespace {
@@ -381,6 +382,10 @@ void DropGraph(pr_gpu_t *h) {
   prgpu::FreeDeviceGraph(&h->g);
 }
 
+unsigned MaxPolls(const pr_gpu_t *h) {
+  return h->wait_polls < 0 ? prgpu::kMaxPolls : static_cast<unsigned>(h->wait_polls);
+}
+
 // Whether a single-column gather solve runs as one resident launch.  It does
 // unless the contribs outgrow what L2 serves well (over 2^23 vertices: 32 MB)
 // and few entries come from the shared-memory tile: then nearly every gather
@@ -462,6 +467,7 @@ int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float da
   a.part = sc.part1;
   a.trace = trace_on_host ? host_trace : sc.trace;
   a.ctl = h->rctl;
+  a.max_polls = MaxPolls(h);
   a.res = h->rres;
   const size_t smem = sizeof(float) * (a.tile + 4);  // and the zero slot
   PR_CHECK(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -471,7 +477,10 @@ int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float da
   PR_CHECK(h, cudaEventRecord(h->ev[3], s));
   PR_CHECK(h, cudaStreamSynchronize(s));
   if (h->rres->failed) {
+    // the sweep that was given up may have counted some segments of a row
     PR_CHECK(h, cudaMemsetAsync(h->rctl, 0, sizeof(prgpu::GridBarrier), s));
+    if (rt.task_start[1])
+      PR_CHECK(h, cudaMemsetAsync(rt.ticket, 0, sizeof(unsigned) * rt.task_start[1], s));
     return SetErr(h, PR_GPU_ECUDA, "a grid barrier of the solve ran out of its wait");
   }
   const int sweeps = h->rres->sweeps;
@@ -1019,7 +1028,8 @@ int pr_gpu_connected_components_device(pr_gpu_t *h, int32_t *comp_out_dev) {
   if (!comp_out_dev) return SetErr(h, PR_GPU_EINVAL, "comp_out is null");
   PR_CHECK(h, cudaSetDevice(h->device));
   std::string msg;
-  cudaError_t e = prgpu::ConnectedComponents(h->g, h->cc, h->stream, comp_out_dev, &msg);
+  cudaError_t e =
+      prgpu::ConnectedComponents(h->g, h->cc, h->stream, MaxPolls(h), comp_out_dev, &msg);
   if (e != cudaSuccess) return SetErr(h, PR_GPU_ECUDA, msg);
   return PR_GPU_OK;
 }
@@ -1035,8 +1045,8 @@ int pr_gpu_bfs_device(pr_gpu_t *h, int64_t source, int32_t *parent_out_dev,
   std::vector<prgpu::BfsStep> log;
   int64_t total = 0;
   cudaError_t e = prgpu::BreadthFirstSearch(h->g, h->bfs, h->stream, static_cast<int>(source), 15,
-                                            18, parent_out_dev, steps ? &log : nullptr, &total,
-                                            &msg);
+                                            18, MaxPolls(h), parent_out_dev,
+                                            steps ? &log : nullptr, &total, &msg);
   if (e != cudaSuccess)
     return SetErr(h, e == cudaErrorMemoryAllocation ? PR_GPU_ENOMEM : PR_GPU_ECUDA, msg);
   int k = 0;
@@ -1354,6 +1364,13 @@ int pr_gpu_sweep_kernel_times(pr_gpu_t *h, int max_iters, double epsilon, double
   if (rc) return rc;
   for (int k = 0; k < h->kernel_n; k++) ms[k] = h->kernel_ms[k];
   if (nkernels) *nkernels = h->kernel_n;
+  return PR_GPU_OK;
+}
+
+int pr_gpu_set_wait_limit(pr_gpu_t *h, int64_t polls) {
+  if (!h) return PR_GPU_EINVAL;
+  if (polls > 0x7fffffffLL) return SetErr(h, PR_GPU_EINVAL, "polls must be below 2^31");
+  h->wait_polls = polls < 0 ? -1 : polls;
   return PR_GPU_OK;
 }
 

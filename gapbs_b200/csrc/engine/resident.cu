@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_solve_kernel(const Resid
       if (lane32 == 0) a.part[gridDim.x + blockIdx.x] = v;  // the slot of odd sweeps
     }
   }
-  if (!grid_barrier(a.ctl, ++round, &s_ok)) {
+  if (!grid_barrier(a.ctl, ++round, a.max_polls, &s_ok)) {
     if (threadIdx.x == 0) a.res->failed = 1;
     return;
   }
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1) resident_solve_kernel(const Resid
       const double v = warp_sum_d(s_red[lane32]);
       if (lane32 == 0) part[blockIdx.x] = v;
     }
-    if (!grid_barrier(a.ctl, ++round, &s_ok)) {
+    if (!grid_barrier(a.ctl, ++round, a.max_polls, &s_ok)) {
       if (threadIdx.x == 0) a.res->failed = 1;
       return;
     }

@@ -16,6 +16,9 @@ constexpr int kResidentThreads = 1024;
 // solve: 88 with 20 CTAs, 96 with 5, 137 with one).
 constexpr int64_t kResidentEntriesPerCta = 1024;
 
+// Polls of a grid barrier before a CTA gives up (about 10 s).
+constexpr unsigned kMaxPolls = 1u << 24;
+
 // State of a barrier between a launch's CTAs (grid_barrier.cuh), zero between
 // launches; a launch whose wait ran out leaves it to be cleared.
 struct GridBarrier {
@@ -61,6 +64,7 @@ struct ResidentArgs {
   double *part;   // 2 x CTAs
   double *trace;  // max_iters
   GridBarrier *ctl;
+  unsigned max_polls;
   ResidentResult *res;
 };
 

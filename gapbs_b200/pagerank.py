@@ -341,6 +341,12 @@ class PageRankEngine:
                     "pr_gpu_sweep_kernel_times")
         return [float(ms[k]) for k in range(nk.value)], int(sw.value)
 
+    def set_wait_limit(self, polls: int = -1):
+        """Polls after which a CTA of a one-launch call gives up waiting for
+        the others and the call fails (pr_gpu_set_wait_limit); negative: the
+        default, about 10 seconds."""
+        self._check(self._lib.pr_gpu_set_wait_limit(self._h, int(polls)), "pr_gpu_set_wait_limit")
+
     def set_stream(self, stream_handle: Optional[int]):
         """Issue work on a caller stream (raw cudaStream_t), None = own stream."""
         self._check(self._lib.pr_gpu_set_stream(self._h, stream_handle), "pr_gpu_set_stream")

@@ -287,6 +287,14 @@ int pr_gpu_sweep_layout_info(pr_gpu_t *h, int *blocked, int *slices, int *bins,
 int pr_gpu_sweep_kernel_times(pr_gpu_t *h, int max_iters, double epsilon, double *ms,
                               int max_kernels, int *nkernels, int32_t *sweeps_out);
 
+/* Limit of the waits inside one-launch calls (gather solves and adjoints,
+ * searches, components), whose CTAs meet at a barrier between their phases:
+ * a CTA that has polled so many times without the others having arrived gives
+ * up, the launch ends, and the call returns PR_GPU_ECUDA with undefined output.
+ * The handle and its graph stay usable.  Negative (the default): about 10
+ * seconds.  No counterpart in the reference. */
+int pr_gpu_set_wait_limit(pr_gpu_t *h, int64_t polls);
+
 /* Makes the handle issue its work on `stream` (a cudaStream_t of the
  * handle's device, e.g. the caller's framework stream) instead of its own;
  * NULL restores the handle's own stream.  The handle does not take
