@@ -40,6 +40,7 @@ namespace prgpu {
 namespace {
 
 constexpr int kThreads = 1024, kCtasPerSm = 2;
+constexpr unsigned kLongList = 32;  // entries of a row that a warp links together
 constexpr int kChaseLimit = 1 << 20;  // far above any tree depth reached
 
 __device__ __forceinline__ int ld_comp(const int *comp, int x) {
@@ -96,7 +97,7 @@ __device__ void cc_link(int u, int v, int *comp, int *err) {
 }
 
 struct CcArgs {
-  int32_t n, active, long_rows;
+  int32_t n, active;
   const int32_t *__restrict__ ooff;
   const int32_t *__restrict__ onbr;
   const int32_t *__restrict__ ioff;  // directed graphs, else null
@@ -165,8 +166,9 @@ __device__ __forceinline__ int compress_one(int v, int *comp, int *err) {
 // Final phase: out-neighbours from the third on and, for a directed graph,
 // all in-neighbours; vertices of the component of row 0 are skipped
 // (src/cc.cc:122-146).  A warp reads the components of 32 consecutive rows at
-// once, since nearly all are skipped, then takes the long rows left (the
-// front of the degree-sorted mirror) together and the others a lane each.
+// once, since nearly all are skipped, then takes the rows left with long lists
+// together and the others a lane each (a lane alone would take a microsecond
+// an entry, and the other CTAs wait at the barrier for at most some seconds).
 __device__ __forceinline__ void link_rest(const CcArgs &a, int giant) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
@@ -174,7 +176,13 @@ __device__ __forceinline__ void link_rest(const CcArgs &a, int giant) {
        b << 5 < a.active; b += warps) {
     const int u = static_cast<int>(b << 5) + lane;
     const bool left = u < a.active && ld_comp(a.comp, u) != giant;
-    unsigned together = __ballot_sync(0xffffffffu, left && u < a.long_rows);
+    // entries of its lists (in- and out-lists of a directed graph differ)
+    unsigned entries = 0;
+    if (left) {
+      entries = a.ooff[u + 1] - a.ooff[u];
+      if (a.ioff) entries += a.ioff[u + 1] - a.ioff[u];
+    }
+    unsigned together = __ballot_sync(0xffffffffu, entries >= kLongList);
     while (together) {
       const int w = static_cast<int>(b << 5) + __ffs(together) - 1;
       together &= together - 1;
@@ -188,7 +196,7 @@ __device__ __forceinline__ void link_rest(const CcArgs &a, int giant) {
       }
       __syncwarp();
     }
-    if (left && u >= a.long_rows) {
+    if (left && entries < kLongList) {
       for (int j = a.ooff[u] + 2; j < a.ooff[u + 1]; j++) cc_link(u, a.onbr[j], a.comp, a.err);
       if (a.ioff)
         for (int j = a.ioff[u]; j < a.ioff[u + 1]; j++) cc_link(u, a.inbr[j], a.comp, a.err);
@@ -294,8 +302,6 @@ cudaError_t ConnectedComponents(const DeviceGraph &g, CcScratch &cs, cudaStream_
   // graph they have no edges at all, so no link ever touches them and they
   // stay their own components: the link and compress passes stop before them.
   a.active = g.directed ? n : static_cast<int32_t>(g.bin_row_start[kBinZero]);
-  // rows of at least 32 entries (the front of the mirror) take a warp each
-  a.long_rows = std::min<int32_t>(a.active, static_cast<int32_t>(g.bin_row_start[4]));
   // out-CSR in new ids: the shared CSR of an undirected graph, the
   // renumbered out-CSR of a directed one
   a.ooff = g.directed ? g.orowoff : g.rowoff;

@@ -382,8 +382,13 @@ void DropGraph(pr_gpu_t *h) {
   prgpu::FreeDeviceGraph(&h->g);
 }
 
+// Polls before a CTA gives up a grid barrier.  The longest work between two
+// barriers that one warp may have alone is a search's or components run's walk
+// of 32 hub rows, at worst nearly all entries of the graph: 16 entries or more
+// a microsecond, and a poll takes about half of one.
 unsigned MaxPolls(const pr_gpu_t *h) {
-  return h->wait_polls < 0 ? prgpu::kMaxPolls : static_cast<unsigned>(h->wait_polls);
+  if (h->wait_polls >= 0) return static_cast<unsigned>(h->wait_polls);
+  return prgpu::kMaxPolls + static_cast<unsigned>(h->g.m / 4);
 }
 
 // Whether a single-column gather solve runs as one resident launch.  It does

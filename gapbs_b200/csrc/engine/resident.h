@@ -16,7 +16,7 @@ constexpr int kResidentThreads = 1024;
 // solve: 88 with 20 CTAs, 96 with 5, 137 with one).
 constexpr int64_t kResidentEntriesPerCta = 1024;
 
-// Polls of a grid barrier before a CTA gives up (about 10 s).
+// Polls of a grid barrier before a CTA gives up (about 10 s), on small graphs.
 constexpr unsigned kMaxPolls = 1u << 24;
 
 // State of a barrier between a launch's CTAs (grid_barrier.cuh), zero between

@@ -344,7 +344,7 @@ class PageRankEngine:
     def set_wait_limit(self, polls: int = -1):
         """Polls after which a CTA of a one-launch call gives up waiting for
         the others and the call fails (pr_gpu_set_wait_limit); negative: the
-        default, about 10 seconds."""
+        default, 10 seconds or more."""
         self._check(self._lib.pr_gpu_set_wait_limit(self._h, int(polls)), "pr_gpu_set_wait_limit")
 
     def set_stream(self, stream_handle: Optional[int]):

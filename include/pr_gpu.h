@@ -292,7 +292,7 @@ int pr_gpu_sweep_kernel_times(pr_gpu_t *h, int max_iters, double epsilon, double
  * a CTA that has polled so many times without the others having arrived gives
  * up, the launch ends, and the call returns PR_GPU_ECUDA with undefined output.
  * The handle and its graph stay usable.  Negative (the default): about 10
- * seconds.  No counterpart in the reference. */
+ * seconds, more on graphs of many entries.  No counterpart in the reference. */
 int pr_gpu_set_wait_limit(pr_gpu_t *h, int64_t polls);
 
 /* Makes the handle issue its work on `stream` (a cudaStream_t of the

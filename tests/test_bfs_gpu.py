@@ -139,6 +139,39 @@ def test_directed_source_without_in_edges(engine):
     assert kinds[1] == "e" and kinds.count("bu") >= 3
 
 
+def test_hub_rows_unreached_bottom_up(engine):
+    """Rows of at least 4,096 in-neighbours that bottom-up steps still have to
+    walk: some with their first frontier entry at the start, inside or at the
+    end of the list, some never reached, over more than one bitmap word."""
+    rng = np.random.default_rng(12)
+    u, v = layered((20000, 30000, 20000), rng, extra=2)
+    n0 = int(v.max()) + 1
+    first = np.arange(n0, n0 + 12000)                        # never reached
+    last = first[-1] + 1 + np.arange(30000)                  # a late layer with large ids
+    layer2 = np.arange(20001, 50001)
+    hubs = last[-1] + 1 + np.arange(70)
+    us, vs = [u, rng.choice(layer2, last.size)], [v, last]
+    want = {}
+    for i, h in enumerate(hubs):
+        src = [rng.choice(first, (4096, 4097, 5000, 8191)[i % 4], replace=False)]
+        if i % 5:                    # 4 of 5 hubs hang on the layer below too
+            src.append(rng.choice(last if i % 2 else layer2, 1 + i % 3, replace=False))
+            want[h] = src[1].min()
+        src = np.concatenate(src)
+        us.append(src)
+        vs.append(np.full(src.size, h))
+    g = Graph.from_edges(np.concatenate(us), np.concatenate(vs), symmetrize=False)
+    assert (np.diff(g.in_offsets) >= 4096).sum() == hubs.size
+    engine.upload(g)
+    parent, steps = engine.bfs(0, with_steps=True)
+    check(g, 0, parent)
+    kinds = [k for k, _, _ in steps]
+    assert "e" in kinds[:3] and kinds.count("bu") >= 3
+    # a bottom-up step takes the first frontier vertex in list order
+    for h in hubs:
+        assert parent[h] == want.get(h, -1)
+
+
 def test_host_stepped_mode_matches(tmp_path):
     # GAPBS_PR_PLAIN_LAUNCH=1 runs the same step kernels launched one by one
     # from the host (the mode profilers use); same trees, same step sequence

@@ -58,6 +58,28 @@ def test_directed_and_adversarial(engine):
         assert np.array_equal(engine.connected_components(), oracle.cc_afforest(g)), name
 
 
+def test_directed_long_out_lists_outside_the_largest(engine):
+    """Rows with few in-edges and long out-lists (and the reverse, and both)
+    outside row 0's component: linked by a warp each; 31 to 33 entries lie at
+    the boundary."""
+    rng = np.random.default_rng(5)
+    us, vs = [np.arange(1, 30000)], [np.zeros(29999, np.int64)]  # row 0: in-degree 29,999
+    base = 30000
+    for k, (out, inn) in enumerate([(20000, 1), (1, 20000), (9000, 9000), (30, 1), (31, 1),
+                                    (32, 1), (17, 15), (17, 16), (0, 33)]):
+        hub = base + rng.integers(0, out + inn + 1)
+        rest = np.setdiff1d(base + np.arange(out + inn + 1), [hub])
+        rng.shuffle(rest)
+        us += [np.full(out, hub), rest[out:]]
+        vs += [rest[:out], np.full(inn, hub)]
+        base += out + inn + 1
+    g = Graph.from_edges(np.concatenate(us), np.concatenate(vs), symmetrize=False)
+    engine.upload(g)
+    comp = engine.connected_components()
+    assert np.array_equal(comp, oracle.cc_afforest(g))
+    assert np.unique(comp).size == 10
+
+
 def test_generated_graph_and_determinism(engine):
     engine.generate("-g 18 -k 4")
     a = engine.connected_components()
