@@ -414,12 +414,4 @@ int BinRowGrid(const SliceBlocks &sb, int64_t n) {
   return sb.nbins + static_cast<int>((n - sb.ndst + zero_rows - 1) / zero_rows);
 }
 
-// contribs + the zero slot, rounded to whole float4
-size_t SliceSmemBytes(const SliceBlocks &sb) { return sizeof(float) * (sb.slice_verts + 4); }
-// the bin's partials, then its positions (16-byte words from the one
-// holding its first position)
-size_t BinSmemBytes(const SliceBlocks &sb) {
-  return sizeof(float) * ((sb.bin_words + 3) & ~3) + sizeof(uint16_t) * (sb.bin_words + 16);
-}
-
 }  // namespace prgpu

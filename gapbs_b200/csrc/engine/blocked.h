@@ -151,8 +151,17 @@ int BinRowThreads(const SliceBlocks &sb);
 constexpr int kSliceThreads = kSliceWarps * 32;
 // Phase-2 grid: the bins, then blocks for the rows without in-edges.
 int BinRowGrid(const SliceBlocks &sb, int64_t n);
-size_t SliceSmemBytes(const SliceBlocks &sb);
-size_t BinSmemBytes(const SliceBlocks &sb);
+// Dynamic shared memory of a launch, and of the largest one: a kernel's limit
+// belongs to the process, so every handle sets the same one.  A slice holds
+// contribs and the zero slot, rounded to whole float4; a bin holds its
+// partials, then its positions (16-byte words from the one holding its first
+// position).
+constexpr size_t SliceSmemBytes(int slice_verts) { return sizeof(float) * (slice_verts + 4); }
+constexpr size_t BinSmemBytes(int bin_words) {
+  return sizeof(float) * ((bin_words + 3) & ~3) + sizeof(uint16_t) * (bin_words + 16);
+}
+constexpr size_t kMaxSliceSmem = SliceSmemBytes(kMaxSliceVerts);
+constexpr size_t kMaxBinSmem = BinSmemBytes(kMaxBinWords);
 
 }  // namespace prgpu
 

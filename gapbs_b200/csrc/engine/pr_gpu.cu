@@ -475,8 +475,9 @@ int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float da
   a.max_polls = MaxPolls(h);
   a.res = h->rres;
   const size_t smem = sizeof(float) * (a.tile + 4);  // and the zero slot
+  // the limit belongs to the process: the same for every handle
   PR_CHECK(h, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem)));
+                                   sizeof(float) * (prgpu::kResidentTile + 4)));
   PR_CHECK(h, cudaEventRecord(h->ev[0], s));
   PR_CHECK(h, prgpu::LaunchGrid(fn, grid, prgpu::kResidentThreads, &a, smem, s));
   PR_CHECK(h, cudaEventRecord(h->ev[3], s));
@@ -630,14 +631,15 @@ int SolveSingle(pr_gpu_t *h, int max_iters, double epsilon, float damping,
     const void *kb = prgpu::BinRowKernel(sb);
     for (const void *k : {kf, kr})
       PR_CHECK(h, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(prgpu::SliceSmemBytes(sb))));
+                                       static_cast<int>(prgpu::kMaxSliceSmem)));
     PR_CHECK(h, cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     static_cast<int>(prgpu::BinSmemBytes(sb))));
+                                     static_cast<int>(prgpu::kMaxBinSmem)));
     for (int i = 0; i < 3; i++) {
       body[i].fn = i == 0 ? kf : (i == 1 ? kr : kb);
       body[i].grid = dim3(i < 2 ? sb.nctas : nblocks);
       body[i].block = dim3(i < 2 ? prgpu::kSliceThreads : prgpu::BinRowThreads(sb));
-      body[i].smem = i < 2 ? prgpu::SliceSmemBytes(sb) : prgpu::BinSmemBytes(sb);
+      body[i].smem = i < 2 ? prgpu::SliceSmemBytes(sb.slice_verts)
+                           : prgpu::BinSmemBytes(sb.bin_words);
       body[i].args = &ba;
       body[i].args_size = sizeof(ba);
       body[i].beside_previous = i == 1;
