@@ -116,7 +116,7 @@ struct Scratch {
   float *base = nullptr;       // per-vertex (1-d) t (PPR), new ids
   float *outbuf = nullptr;     // n x ncols scores in original ids
   float *tele = nullptr;       // teleport staging (original ids)
-  float *aux = nullptr;        // adjoint: forward scores staging (original ids)
+  float *aux = nullptr;        // adjoint: forward scores (original ids), staged or copied
   float *edge_buf = nullptr;   // adjoint: m edge gradients (device staging)
   double *norm = nullptr;      // adjoint: ||w||_1
   int64_t cap_edges = 0;

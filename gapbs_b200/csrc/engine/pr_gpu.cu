@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <limits>
 #include <memory>
 #include <mutex>
@@ -711,10 +712,23 @@ int SolveSingle(pr_gpu_t *h, int max_iters, double epsilon, float damping,
 }
 
 
-// Adjoint solve on device buffers (original ids in, original ids out).
+bool Overlap(const float *a, int64_t na, const float *b, int64_t nb) {
+  return a && b && std::less<const float *>()(a, b + nb) && std::less<const float *>()(b, a + na);
+}
+
+// Adjoint solve on device buffers (original ids in, original ids out).  The
+// outputs may overlap the inputs: loss_w is read before either is written, and
+// of scores that lie where an output goes the gradients read a copy.
 int SolveAdjoint(pr_gpu_t *h, int max_iters, double epsilon, float damping, const float *w_old,
                  const float *s_old, float *grad_t_old, float *grad_ew) {
   DeviceGraph &g = h->g;
+  if (Overlap(s_old, g.n, grad_t_old, g.n) || Overlap(s_old, g.n, grad_ew, g.m)) {
+    int rc = EnsureScratch(h, g.n, 1, 1, max_iters);
+    if (rc) return rc;
+    PR_CHECK(h, cudaMemcpyAsync(h->sc.aux, s_old, sizeof(float) * g.n, cudaMemcpyDeviceToDevice,
+                                h->stream));
+    s_old = h->sc.aux;
+  }
   if (UseResident(h, prgpu::kKindAdjoint)) {
     int rc = SolveResident(h, prgpu::kKindAdjoint, max_iters, epsilon, damping, w_old, grad_t_old,
                            &h->last_adjoint_sweeps, nullptr);

@@ -189,7 +189,8 @@ int pr_gpu_adjoint(pr_gpu_t *h, int max_iters, double epsilon, float damping,
                    float *grad_teleport, float *grad_edge_w,
                    int32_t *sweeps_out);
 
-/* Device-pointer form of pr_gpu_adjoint (no counterpart in the reference). */
+/* Device-pointer form of pr_gpu_adjoint (no counterpart in the reference).
+ * Either output may take the place of an input. */
 int pr_gpu_adjoint_device(pr_gpu_t *h, int max_iters, double epsilon,
                           float damping, const float *loss_w_dev,
                           const float *scores_dev, float *grad_teleport_dev,

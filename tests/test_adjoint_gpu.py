@@ -155,3 +155,47 @@ def test_autograd_training_loop_updates_weights_on_device(engine):
                                rowsum=row_sums(g, ew), max_iters=2000, epsilon=1e-14)
     assert np.abs(s.detach().cpu().numpy() - s64).sum() <= 1e-5
     pctx.engine.close()
+
+
+@pytest.mark.parametrize("kind", ["undirected", "directed", "weighted", "large_uniform"])
+def test_outputs_in_place_of_inputs(engine, kind):
+    """Gradients written over loss_w or scores are those written elsewhere:
+    the edge gradients read the scores after the teleport gradient is done."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(23)
+    if kind == "directed":
+        g = Graph.from_edges(rng.integers(0, 3000, 30000), rng.integers(0, 3000, 30000))
+    elif kind == "large_uniform":   # the sweep launches
+        u, v = rng.integers(0, (1 << 23) + 5, (2, 1 << 24), dtype=np.int32)
+        g = Graph.from_edges(u, v, symmetrize=True)
+    else:
+        g = make_graph("-g 12")
+    n, m = g.num_nodes, g.num_edges_directed
+    ew = rng.uniform(0.5, 1.5, m).astype(np.float32) if kind == "weighted" else None
+    engine.upload(g, edge_w=ew)
+    w = torch.from_numpy(rng.normal(size=n).astype(np.float32)).cuda()
+    s = torch.from_numpy(rng.random(n).astype(np.float32) / n).cuda()
+
+    def grads(w, s, gt, ge):
+        torch.cuda.synchronize()
+        engine.adjoint_device(5, 0.0, 0.85, w.data_ptr(), s.data_ptr(), gt.data_ptr(),
+                              ge.data_ptr())
+        return gt, ge
+
+    gt, ge = grads(w, s, torch.empty(n, device="cuda"), torch.empty(m, device="cuda"))
+    assert float(ge.abs().max()) > 0
+    s1 = s.clone()
+    a, b = grads(w, s1, s1, torch.empty(m, device="cuda"))       # teleport over scores
+    assert torch.equal(a, gt) and torch.equal(b, ge)
+    w1 = w.clone()
+    a, b = grads(w1, s, w1, torch.empty(m, device="cuda"))       # teleport over loss_w
+    assert torch.equal(a, gt) and torch.equal(b, ge)
+    for first in (0, m - n):                                     # edges over scores
+        buf = torch.empty(m, device="cuda")
+        buf[first:first + n] = s
+        a, b = grads(w, buf[first:first + n], torch.empty(n, device="cuda"), buf)
+        assert torch.equal(a, gt) and torch.equal(b, ge)
+    buf = torch.empty(n + 8, device="cuda")                      # partly over scores
+    buf[8:] = s
+    a, b = grads(w, buf[8:], buf[:n], torch.empty(m, device="cuda"))
+    assert torch.equal(a, gt) and torch.equal(b, ge)
