@@ -423,8 +423,8 @@ int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float da
   prgpu::ResidentArgs a;
   std::memset(&a, 0, sizeof(a));
   a.tile = static_cast<int32_t>(std::min<int64_t>(g.n, prgpu::kResidentTile) & ~int64_t(3));
-  const int grid = static_cast<int>(
-      std::max<int64_t>(1, std::min<int64_t>(sms, g.m / prgpu::kResidentEntriesPerCta)));
+  const int grid = static_cast<int>(std::max<int64_t>(
+      1, std::min<int64_t>(sms, std::max(g.m, g.n) / prgpu::kResidentEntriesPerCta)));
   int rc = EnsureScratch(h, g.n, 1, 2 * grid, max_iters);
   if (rc) return rc;
   Scratch &sc = h->sc;

@@ -131,3 +131,22 @@ def test_large_uniform_graph_keeps_sweep_launches(engine):
                                               epsilon=0.0)
     assert np.linalg.norm(gt - gt64) <= 1e-4 * np.linalg.norm(gt64)
     assert np.linalg.norm(ge - gw64) <= 1e-3 * np.linalg.norm(gw64)
+
+
+def test_many_vertices_few_edges(engine):
+    """Init, sweeps and write-back of a graph with hardly any edges use the
+    whole GPU: 16 M vertices pass through DRAM a few times, well under a
+    millisecond (several with a CTA per 1,024 entries, a few SMs only)."""
+    n = 1 << 24
+    rng = np.random.default_rng(10)
+    u, v = rng.integers(0, n, (2, 3000), dtype=np.int32)
+    u[0] = n - 1
+    g = Graph.from_edges(u, v, symmetrize=True)
+    engine.upload(g)
+    check(engine, g)
+    ms = []
+    for _ in range(5):
+        engine.run(20, 1e-4)
+        ms.append(engine.last_timing()[1])
+    print("device ms a solve:", ms)
+    assert min(ms) < 1.5
