@@ -333,6 +333,7 @@ def run_ours(a, dist: Dist):
     # the sweep layout the timed solves ran with
     layout = eng.sweep_layout_info()
     blocked = layout["last_run_blocked"]
+    one_launch = launches == a.steps  # gather solves, each a launch
 
     # ---- end to end through the C-ABI host call (pinned host result buffer)
     eng.set_stream(None)
@@ -421,7 +422,7 @@ def run_ours(a, dist: Dist):
         bfs = {"workload": f"direction-optimizing BFS of {a.graph.strip()} from {len(picked)} "
                            "sources with out-edges (seeded draw)",
                "ms": round(bfs_ms, 3), "unit": "ms per search (device-resident graph, one "
-                                               "graph launch per search)",
+                                               "launch per search)",
                "gteps": round(m / (bfs_ms / 1e3) / 1e9, 2), "steps_per_search":
                    round(steps_total / max(1, len(picked)), 1), "sources": picked}
         eng.set_stream(None)
@@ -468,13 +469,15 @@ def run_ours(a, dist: Dist):
     bps = sweep_bytes(n, m, directed)
     avg_sweep_ms = sweep_ms_total / max(sweeps_total, 1)
     achieved = bps / (avg_sweep_ms / 1e3) / 1e9
-    traffic = profiled_traffic(a.graph, blocked)
-    # each kernel of the sweep body timed on its own (CUDA events between
-    # separate launches, one extra solve outside the timed region)
+    traffic = None if one_launch else profiled_traffic(a.graph, blocked)
+    # each kernel of the sweep timed on its own, in one extra solve outside the
+    # timed region: CUDA events between separate launches, or, where a solve is
+    # one launch, the device's clock from the first sweep to the last
     kms, ksweeps = eng.sweep_kernel_times(a.max_iters, a.epsilon)
     assert len(kms) == (3 if blocked else 1), "sweep layout changed between legs"
     knames = (["slice_partial_kernel<flat pairs>", "slice_partial_kernel<other pairs>",
-               "bin_row_kernel"] if blocked else ["pull_sweep_kernel"])
+               "bin_row_kernel"] if blocked
+              else ["resident_solve_kernel" if one_launch else "pull_sweep_kernel"])
     kernels = [{"kernel": kn, "ms_per_sweep": round(t, 4), "share": round(t / sum(kms), 4)}
                for kn, t in zip(knames, kms)]
     if blocked:
@@ -532,7 +535,7 @@ def run_ours(a, dist: Dist):
         },
         "roofline": {
             "kernel": ("slice-blocked sweep: " + ", ".join(knames) + " (one launch each per "
-                       "sweep)") if blocked else "pull_sweep_kernel",
+                       "sweep)") if blocked else knames[0],
             "bound": "hbm",
             "achieved": round(achieved, 1),
             "peak": peak,
@@ -543,9 +546,11 @@ def run_ours(a, dist: Dist):
             "algorithmic_bytes_per_sweep": bps,
             "avg_sweep_ms": round(avg_sweep_ms, 4),
             "kernels": kernels,
-            "kernels_note": "average device ms per sweep of each kernel, each launched on its "
-                            f"own between CUDA events ({ksweeps} sweeps, one solve outside the "
-                            "timed region)",
+            "kernels_note": "average device ms per sweep of each kernel, "
+                            + ("from the first sweep to the last of the one launch "
+                               if one_launch else
+                               "each launched on its own between CUDA events ")
+                            + f"({ksweeps} sweeps, one solve outside the timed region)",
             "layout_bytes_per_sweep": int(layout_bytes),
             "layout_gbs": round(layout_bytes / (avg_sweep_ms / 1e3) / 1e9, 1),
             "layout_frac": round(layout_bytes / (avg_sweep_ms / 1e3) / 1e9 / peak, 4),

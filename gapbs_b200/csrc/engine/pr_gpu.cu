@@ -49,8 +49,8 @@ struct pr_gpu {
   int64_t last_launches = 0;
   int last_adjoint_sweeps = 0;
   bool last_blocked = false;
-  // pr_gpu_sweep_kernel_times: per-kernel events of one timed solve and the
-  // average device ms per sweep of each kernel of the sweep body
+  // pr_gpu_sweep_kernel_times: per-kernel events of one timed solve of several
+  // launches, and the average device ms per sweep of each kernel of the sweep
   bool time_kernels = false;
   std::vector<cudaEvent_t> kev;
   double kernel_ms[3] = {0, 0, 0};
@@ -501,6 +501,10 @@ int SolveResident(pr_gpu_t *h, int kind, int max_iters, double epsilon, float da
   float ms_total = 0;
   cudaEventElapsedTime(&ms_total, h->ev[0], h->ev[3]);
   h->last_sweep_ms = h->rres->sweep_ns * 1e-6;
+  if (h->time_kernels) {
+    h->kernel_n = 1;
+    h->kernel_ms[0] = sweeps ? h->last_sweep_ms / sweeps : 0.0;
+  }
   h->last_total_ms = ms_total;
   h->last_launches = 1;
   h->last_blocked = false;
@@ -525,7 +529,7 @@ int SolveSingle(pr_gpu_t *h, int max_iters, double epsilon, float damping,
                   "source slices than a bin holds)");
   const bool blocked = UseBlocked(h);
   const int kind = tele_old ? prgpu::kKindPPR : prgpu::kKindPlain;
-  if (!blocked && !h->time_kernels && UseResident(h, kind))
+  if (!blocked && UseResident(h, kind))
     return SolveResident(h, kind, max_iters, epsilon, damping, tele_old, out_old, sweeps_out,
                          err_trace);
   int32_t task_start[prgpu::kNumBins + 1];

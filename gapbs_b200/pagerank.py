@@ -331,9 +331,9 @@ class PageRankEngine:
         return err.value
 
     def sweep_kernel_times(self, max_iters: int = 20, epsilon: float = 1e-4):
-        """One plain solve with every sweep kernel timed on its own
-        (pr_gpu_sweep_kernel_times): the average device ms per sweep of each
-        kernel of the sweep body in launch order, and the sweep count."""
+        """One plain solve (pr_gpu_sweep_kernel_times): the average device ms
+        per sweep of each kernel that its sweeps are made of, in launch order,
+        and the sweep count."""
         ms = (c_double * 3)()
         nk, sw = c_int(), c_int32()
         self._check(self._lib.pr_gpu_sweep_kernel_times(self._h, int(max_iters), float(epsilon),

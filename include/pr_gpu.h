@@ -238,15 +238,18 @@ int pr_gpu_get_batch_schedule(const pr_gpu_t *h, int *width, int *short_len, int
 /* Sweep layout of single-column solves (plain and personalized PageRank) on
  * unweighted graphs:
  *   PR_GPU_SWEEP_AUTO     slice-blocked when the graph has at least 48 Mi
- *                         (48 x 2^20) edges (below that the gather sweep's
- *                         contribs stay in the caches), fits that layout's
+ *                         (48 x 2^20) edges (below that a gather solve is as
+ *                         fast or faster), fits that layout's
  *                         limits, the device has room for it and its
  *                         in-edges form at most M/2 (row, slice) pairs
  *                         (skewed graphs such as Kronecker ones; on uniform
  *                         random graphs nearly every edge is a pair of its
  *                         own and gather is faster), else gather
- *   PR_GPU_SWEEP_GATHER   one sweep kernel that gathers contrib[v] for every
- *                         in-edge (no extra device memory)
+ *   PR_GPU_SWEEP_GATHER   sweeps that gather contrib[v] for every in-edge (no
+ *                         extra device memory): the whole solve is one launch,
+ *                         except on graphs of over 2^23 vertices with few of
+ *                         their entries from the highest in-degrees (uniform
+ *                         ones), where each sweep is a launch
  *   PR_GPU_SWEEP_BLOCKED  slice-blocked; a run on a graph it does not fit
  *                         returns PR_GPU_EINVAL
  * The slice-blocked sweep is three kernels per sweep: per slice of
@@ -276,15 +279,16 @@ int pr_gpu_sweep_layout_info(pr_gpu_t *h, int *blocked, int *slices, int *bins,
                              int *last_blocked);
 
 /* Measurement aid: runs one plain PageRank solve of the uploaded graph
- * (uniform teleport, damping 0.85; scores left in an internal buffer) with
- * every sweep kernel launched on its own between CUDA events on the
- * handle's stream, and writes the average device time per sweep of each
- * kernel of the sweep body, in launch order, to ms[0 .. *nkernels):
- * slice-blocked: flat-pair partials, other partials, row update; gather:
- * the sweep kernel.  max_kernels: room in ms (at least 3).  *sweeps_out:
- * the sweeps the solve ran.  The timings include no loop or launch
- * overhead of the regular CUDA-graph loop.  No counterpart in the
- * reference. */
+ * (uniform teleport, damping 0.85; scores left in an internal buffer) and
+ * writes the average device time per sweep of each kernel of the sweep, in
+ * launch order, to ms[0 .. *nkernels).  Slice-blocked (flat-pair partials,
+ * other partials, row update) and gather sweeps that are a launch each (the
+ * sweep kernel): every kernel launched on its own between CUDA events on the
+ * handle's stream, without the loop and launch overhead of the regular
+ * CUDA-graph loop.  A gather solve in one launch: its time from the first
+ * sweep to the last, by the device's clock, over the sweeps (barriers
+ * included).  max_kernels: room in ms (at least 3).  *sweeps_out: the sweeps
+ * the solve ran.  No counterpart in the reference. */
 int pr_gpu_sweep_kernel_times(pr_gpu_t *h, int max_iters, double epsilon, double *ms,
                               int max_kernels, int *nkernels, int32_t *sweeps_out);
 
@@ -302,8 +306,9 @@ int pr_gpu_set_wait_limit(pr_gpu_t *h, int64_t polls);
  * ownership.  Calls still synchronize that stream before returning. */
 int pr_gpu_set_stream(pr_gpu_t *h, void *stream);
 
-/* Device time (CUDA events on the handle's stream) of the sweep kernels of
- * the last run and the number of engine kernel launches it made. */
+/* Device time of the last run: of its sweeps (CUDA events around them on the
+ * handle's stream; in a solve of one launch the device's own clock), of the
+ * whole run (CUDA events), and the number of engine kernel launches it made. */
 int pr_gpu_last_timing(const pr_gpu_t *h, double *sweep_ms, double *total_ms,
                        int64_t *kernel_launches);
 

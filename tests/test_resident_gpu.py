@@ -150,3 +150,15 @@ def test_many_vertices_few_edges(engine):
         ms.append(engine.last_timing()[1])
     print("device ms a solve:", ms)
     assert min(ms) < 1.5
+
+
+def test_kernel_times_are_of_the_solve_that_runs(engine):
+    """pr_gpu_sweep_kernel_times on the gather layout times the one launch that
+    ordinary solves are."""
+    engine.upload(make_graph("-g 16"))
+    res = engine.run(20, 1e-4)
+    assert engine.last_timing()[2] == 1
+    ms, sweeps = engine.sweep_kernel_times(20, 1e-4)
+    sweep_ms, total_ms, launches = engine.last_timing()
+    assert launches == 1 and len(ms) == 1 and sweeps == int(res.sweeps[0])
+    assert 0 < ms[0] * sweeps <= total_ms and ms[0] * sweeps == pytest.approx(sweep_ms)
