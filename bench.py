@@ -296,7 +296,11 @@ def run_ours(a, dist: Dist):
         eng.upload(g)
         upload_s = time.perf_counter() - t0
         upload_bytes = 4 * (n + 1) + 4 * m
-    stream = torch.cuda.current_stream(dev)
+    # a stream of its own for the bench and the engine: a handle given the
+    # default stream issues on its own one, beside the buffer write that evicts
+    # L2, and the events around a step would not be on the launching stream
+    stream = torch.cuda.Stream(dev)
+    torch.cuda.set_stream(stream)
     eng.set_stream(stream.cuda_stream)
     out = torch.empty(n, dtype=torch.float32, device=f"cuda:{dev}")
     flush = torch.empty(64 * 1024 * 1024, dtype=torch.float32, device=f"cuda:{dev}")  # 256 MB > L2
