@@ -35,7 +35,10 @@ class PageRankContext:
     adjoint_max_iters: int = 300
     adjoint_epsilon: float = 1e-6
     engine: PageRankEngine = field(init=False)
-    _weights_key: Optional[tuple] = field(default=None, init=False)
+    # what the engine holds: (key, tensor) of the weights, (None, None) for unit
+    # ones.  The tensor is kept, so that no other can take its address and pass
+    # for it.
+    _weights: Optional[tuple] = field(default=None, init=False)
     last_sweeps: int = field(default=0, init=False)
     last_adjoint_sweeps: int = field(default=0, init=False)
     uploads: int = field(default=0, init=False)          # full graph uploads
@@ -48,10 +51,10 @@ class PageRankContext:
         """Puts edge_w (or unit weights for None) in the engine: a full
         upload the first time and when switching between weighted and
         unweighted, else a device-to-device weight update."""
-        key = None if edge_w is None else (edge_w.data_ptr(), edge_w._version, edge_w.numel())
-        if self._weights_key is not None and key == self._weights_key[0]:
+        key = _weights_key(edge_w)
+        if self._weights is not None and key == self._weights[0]:
             return
-        was_weighted = self._weights_key is not None and self._weights_key[0] is not None
+        was_weighted = self._weights is not None and self._weights[0] is not None
         if edge_w is not None and was_weighted:
             if edge_w.numel() != self.engine.m:
                 raise ValueError("edge_w must have one entry per directed edge")
@@ -63,7 +66,14 @@ class PageRankContext:
             w = None if edge_w is None else edge_w.detach().float().cpu().numpy()
             self.engine.upload(self.graph, edge_w=w)
             self.uploads += 1
-        self._weights_key = (key,)
+        self._weights = (key, None if edge_w is None else edge_w.detach())
+
+
+def _weights_key(w: Optional[torch.Tensor]):
+    """Equal for tensors of equal contents as long as the first is alive."""
+    if w is None:
+        return None
+    return (w.data_ptr(), w._version, w.dtype, tuple(w.shape), w.stride())
 
 
 def _cuda_f32(x: torch.Tensor, dev: int) -> torch.Tensor:

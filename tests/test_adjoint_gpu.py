@@ -199,3 +199,35 @@ def test_outputs_in_place_of_inputs(engine, kind):
     buf[8:] = s
     a, b = grads(w, buf[8:], buf[:n], torch.empty(m, device="cuda"))
     assert torch.equal(a, gt) and torch.equal(b, ge)
+
+
+def test_autograd_fresh_weight_tensors():
+    """Weights that are a new tensor every step, in memory that the last one
+    left, or another view of the same memory: each solve takes its own."""
+    torch = pytest.importorskip("torch")
+    if not gpu_available():
+        pytest.skip("no CUDA device")
+    from gapbs_b200.autograd import PageRankContext, personalized_pagerank
+    rng = np.random.default_rng(9)
+    g = make_graph("-g 11")
+    n, m = g.num_nodes, g.num_edges_directed
+    kw = dict(max_iters=100, epsilon=1e-7)
+    t = torch.from_numpy(seed_teleports(g, 1, rng)[:, 0]).cuda()
+    host = [torch.from_numpy(rng.uniform(0.5, 1.5, m).astype(np.float32)) for _ in range(3)]
+
+    def alone(w):
+        pctx = PageRankContext(g, **kw)
+        return personalized_pagerank(t, w, pctx).clone()
+
+    want = [alone(w.cuda()) for w in host]
+    pctx = PageRankContext(g, **kw)
+    for w, expect in zip(host, want):
+        d = w.cuda()
+        assert torch.equal(personalized_pagerank(t, d, pctx), expect)
+        del d                                    # its memory is free again
+    both = torch.empty(2 * m, device="cuda")     # one address, two strides
+    both[0::2], both[m:] = host[0].cuda(), 1.0
+    even, front = both[0::2], both[:m]
+    assert even.data_ptr() == front.data_ptr()
+    for w in (even, front):
+        assert torch.equal(personalized_pagerank(t, w, pctx), alone(w.contiguous()))
