@@ -96,6 +96,7 @@ class PageRankFunction(torch.autograd.Function):
         pctx.last_sweeps = int(sweeps[0])
         ctx.pctx = pctx
         ctx.has_w = edge_w is not None
+        ctx.weights = pctx._weights
         ctx.save_for_backward(out)
         return out
 
@@ -104,6 +105,12 @@ class PageRankFunction(torch.autograd.Function):
         (s,) = ctx.saved_tensors
         pctx: PageRankContext = ctx.pctx
         eng = pctx.engine
+        key, held = ctx.weights
+        if pctx._weights[0] != key:   # another forward pass came between
+            if _weights_key(held) != key:
+                raise RuntimeError("the edge weights of this pass were changed in place and the "
+                                   "engine holds others since")
+            pctx.ensure_weights(held)
         gs = _cuda_f32(grad_s, pctx.device)
         grad_t = torch.empty(eng.n, device=gs.device, dtype=torch.float32)
         want_w = ctx.has_w and ctx.needs_input_grad[1]

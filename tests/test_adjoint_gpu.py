@@ -231,3 +231,48 @@ def test_autograd_fresh_weight_tensors():
     assert even.data_ptr() == front.data_ptr()
     for w in (even, front):
         assert torch.equal(personalized_pagerank(t, w, pctx), alone(w.contiguous()))
+
+
+def test_autograd_backward_uses_its_own_weights():
+    """Two forward passes with different weights on one context, then both
+    backward passes: each has the gradients that it has alone.  Weights changed
+    in place after a pass: its gradients while the engine still holds the old
+    ones, an error once it does not."""
+    torch = pytest.importorskip("torch")
+    if not gpu_available():
+        pytest.skip("no CUDA device")
+    from gapbs_b200.autograd import PageRankContext, personalized_pagerank
+    rng = np.random.default_rng(10)
+    g = make_graph("-g 11")
+    n, m = g.num_nodes, g.num_edges_directed
+    kw = dict(max_iters=100, epsilon=1e-7)
+    t = torch.from_numpy(seed_teleports(g, 1, rng)[:, 0]).cuda().requires_grad_()
+    lw = torch.from_numpy(rng.normal(size=n).astype(np.float32)).cuda()
+    weights = [torch.from_numpy(rng.uniform(0.5, 1.5, m).astype(np.float32)).cuda()
+               .requires_grad_() for _ in range(2)] + [None]
+
+    def loss(w, pctx):
+        return (lw * personalized_pagerank(t, w, pctx)).sum()
+
+    def grads(value, w):
+        return torch.autograd.grad(value, (t,) if w is None else (t, w))
+
+    def alone(w):
+        return grads(loss(w, PageRankContext(g, **kw)), w)
+
+    pctx = PageRankContext(g, **kw)
+    want = [alone(w) for w in weights]
+    values = [loss(w, pctx) for w in weights]
+    for value, w, expect in zip(values, weights, want):
+        assert all(torch.equal(a, b) for a, b in zip(grads(value, w), expect))
+    a, b = weights[:2]
+    value = loss(a, pctx)
+    with torch.no_grad():
+        a.mul_(2.0)
+    assert all(torch.equal(x, y) for x, y in zip(grads(value, a), want[0]))
+    value = loss(b, pctx)
+    with torch.no_grad():
+        b.mul_(2.0)
+    loss(a, pctx)
+    with pytest.raises(RuntimeError, match="changed in place"):
+        grads(value, b)
