@@ -358,10 +358,9 @@ int EnsureSliceBlocks(pr_gpu_t *h) {
   h->sb_built = true;
   h->loop_blocked.Reset();
   std::string msg;
-  // below about 48 M edges a resident gather solve is faster (Kronecker 2^20,
-  // 31 M edges: 0.54 ms a solve against 1.0; 2^21, 64 M edges: 0.95 against
-  // 1.09; 3 M vertices, 76 M edges: 1.42 / 1.47; 2^22, 128 M edges: 1.96 /
-  // 1.67 -- the sizes between keep the layout, as documented in pr_gpu.h)
+  // a resident gather solve against a slice-blocked one, ms (Kronecker): 2^20
+  // vertices, 31 M edges 0.55 / 0.59; 2^21, 64 M edges 0.95 / 0.73; 2^22,
+  // 128 M edges 1.96 / 1.25
   if (h->sweep_layout == PR_GPU_SWEEP_AUTO && h->g.m < kAutoBlockedMinEdges) return PR_GPU_OK;
   const int64_t max_pairs = h->sweep_layout == PR_GPU_SWEEP_AUTO
                                 ? h->g.m / 2
@@ -396,10 +395,13 @@ unsigned MaxPolls(const pr_gpu_t *h) {
 // unless the contribs outgrow what L2 serves well (over 2^23 vertices: 32 MB)
 // and few entries come from the shared-memory tile: then nearly every gather
 // waits on L2 or HBM, and the sweep kernel's larger number of resident warps
-// hides that better (uniform graphs, degree 32, ms a solve, resident against
-// sweep launches: 2^22 vertices 3.4 / 3.7, 2^24 17.5 / 15.5; Kronecker 2^23
-// 4.3 / 6.1).  The adjoint of a directed graph, whose out-rows have no
-// order by length, always does.
+// hides that better.  Measured, ms, resident / sweep launches: uniform solves
+// 2^22 vertices 3.4 / 3.7, 2^23 6.7 / 7.4 (degree 32; 4.8 / 5.1 at 16, 10.8 /
+// 12.3 at 64), 2^24 17.5 / 15.5; Kronecker solves 2^22 2.0 / 2.9, 2^23 4.4 /
+// 6.4, 2^24 9.9 / 12.1, 2^25 21.2 / 26.4; eight weighted sweeps, Kronecker 2^23
+// 6.1 / 8.4, 2^24 12.8 / 16.1, uniform 2^23 10.6 / 11.1; six adjoint sweeps,
+// Kronecker 2^24 8.7 / 12.8, uniform 2^23 6.8 / 8.6.  The adjoint of a
+// directed graph, whose out-rows have no order by length, always does.
 bool UseResident(const pr_gpu_t *h, int kind) {
   const DeviceGraph &g = h->g;
   if (kind == prgpu::kKindAdjoint && g.directed) return true;

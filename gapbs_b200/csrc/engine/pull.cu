@@ -294,7 +294,8 @@ pull_sweep_kernel(const PullArgs a) {
 // written by T threads (a warp, or a block for the long rows):
 //   (P lambda)[v] = sum_e w_e lambda[u_e] / S_v
 //   grad_ew[orig position of e] = d s[v] / S_v (lambda[u_e] - (P lambda)[v])
-// Rows of at least 1,024 entries get a block of 1,024 threads each: one warp
+// Rows cut into segments by the solves (at least 1,024 entries, 2,048 on large
+// unweighted graphs) get a block of 1,024 threads each: one warp
 // takes 60,000 entries (the longest row of a Kronecker 2^20 graph) in 1,900
 // dependent rounds, twice (whole pass 536 us; 423 us with blocks).
 struct GradArgs {
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(1024) edge_grad_long_kernel(const GradArgs a) 
   edge_grad_row<1024>(a, blockIdx.x, threadIdx.x, sred);
 }
 
-// Positions [first, end): rows with entries, below 1,024.
+// Positions [first, end): the shorter rows with entries.
 __global__ void __launch_bounds__(256)
 edge_grad_kernel(const GradArgs a, int32_t first, int32_t end) {
   const int64_t p = first + ((static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) >> 5);
