@@ -148,8 +148,10 @@ noalloc_sweep_kernel(unsigned char *scratch, int32_t n, const int32_t *__restric
   for (int u = blockIdx.x * (kNoAllocThreads / 32) + (threadIdx.x >> 5); u < n; u += warps) {
     const int rs = in_off[u], re = in_off[u + 1];
     float acc = 0.f;
-    const unsigned end = re;  // e + 32 may pass 2^31
-    for (unsigned e = rs + lane; e < end; e += 32) acc = __fadd_rn(acc, cin[in_nbr[e]]);
+    // 64 bits: e + 32 may pass 2^31 (an unsigned count keeps the compiler from
+    // unrolling: 13.9 ms a solve of Kronecker 2^20 against 10.0)
+    for (int64_t e = static_cast<int64_t>(rs) + lane; e < re; e += 32)
+      acc = __fadd_rn(acc, cin[in_nbr[e]]);
     acc = warp_sum_f(acc);
     if (lane == 0) {
       const float old = score[u];
