@@ -200,11 +200,10 @@ def measured_peak():
     return HBM_FALLBACK_GBS, "fallback"
 
 
-def profiled_traffic(graph_args: str, blocked: bool):
-    """DRAM bytes per sweep (all kernels of one sweep) from the committed ncu
-    summary of the sweep layout in use."""
-    name = "blocked_sweep_traffic.json" if blocked else "pull_sweep_traffic.json"
-    p = os.path.join(ROOT, "profiles", name)
+def profiled_traffic(graph_args: str):
+    """DRAM bytes per slice-blocked sweep (its three kernels) from the committed
+    ncu summary."""
+    p = os.path.join(ROOT, "profiles", "blocked_sweep_traffic.json")
     if not os.path.exists(p):
         return None
     with open(p) as fh:
@@ -473,7 +472,7 @@ def run_ours(a, dist: Dist):
     bps = sweep_bytes(n, m, directed)
     avg_sweep_ms = sweep_ms_total / max(sweeps_total, 1)
     achieved = bps / (avg_sweep_ms / 1e3) / 1e9
-    traffic = None if one_launch else profiled_traffic(a.graph, blocked)
+    traffic = profiled_traffic(a.graph) if blocked else None
     # each kernel of the sweep timed on its own, in one extra solve outside the
     # timed region: CUDA events between separate launches, or, where a solve is
     # one launch, the device's clock from the first sweep to the last
